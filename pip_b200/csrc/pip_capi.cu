@@ -630,7 +630,8 @@ int pip_ctx_create(const pip_params *p, pip_ctx **out) {
   c->dz.assign(p->dz, p->dz + p->kx);
   c->p.dx = c->p.dy = c->p.dz = nullptr;
   build_kparams(c);
-  c->L = p->fp_exact ? &pip::launchers_exact() : &pip::launchers_fast();
+  c->L = p->fp_exact ? &pip::launchers_exact()
+                     : p->flag_heat == 1 ? &pip::launchers_heat() : &pip::launchers_fast();
   c->mixed = p->precision == PIP_MIXED;
   auto fail = [&](cudaError_t e) {
     g_last_cuda_error = (int)e;

@@ -103,7 +103,7 @@ struct DevCtrl {
   unsigned int blocks_done;       // last-block-done counter of the stage-2 kernel
 };
 
-// Host launchers (one set per arithmetic flavour: FMA-contracted or FMA-free).
+// Host launchers (one set per arithmetic flavour).
 struct Launchers {
   cudaError_t (*prepare)();
   // tm: the TMA map of Us for the 2D tiles (tile_map), or null for per-thread loads.  rows
@@ -139,6 +139,7 @@ struct Launchers {
 };
 
 const Launchers &launchers_fast();
+const Launchers &launchers_heat();   // contexts with conduction: see pip_fp64_heat.cu
 const Launchers &launchers_exact();
 
 }  // namespace pip

@@ -1,6 +1,11 @@
-// pip_step_impl.cuh -- FP64 kernels of the two-fluid step.  Included by pip_fp64_fast.cu
-// (FMA contraction on) and pip_fp64_exact.cu (-fmad=false, bitwise comparable with the
-// CPU restatement); PIP_FLAVOUR names the namespace and PIP_LAUNCHERS the table getter.
+// pip_step_impl.cuh -- FP64 kernels of the two-fluid step, in three flavours:
+//   pip_fp64_fast.cu   FMA contraction, PIP_RCP and PIP_FAST: the forms of
+//                      pip_fp64_forms.cuh (the default build)
+//   pip_fp64_heat.cu   FMA contraction, PIP_RCP: the reciprocal forms of pip_physics.cuh, for
+//                      contexts with implicit conduction (see launch_stage)
+//   pip_fp64_exact.cu  -fmad=false: the literal forms, bitwise comparable with the CPU
+//                      restatement
+// PIP_FLAVOUR names the namespace and PIP_LAUNCHERS the table getter.
 //
 // Layout in HBM: one array of NV = nvm + 5 planes, each plane the Fortran
 // (ix,jx) slab with ghosts (x fastest): ion planes 0..nvm-1 (ro, mx, my, mz, en, bx, by,
@@ -10,9 +15,15 @@
 
 #include <cstring>
 
+#include "pip_fp64_forms.cuh"
 #include "pip_kernels.cuh"
 #include "pip_physics.cuh"
 #include "pip_tma.cuh"
+
+// 1: the flavour of conduction contexts, 2D without resistivity
+#ifndef PIP_HEAT_ONLY
+#define PIP_HEAT_ONLY 0
+#endif
 
 namespace pip {
 namespace PIP_FLAVOUR {
@@ -55,7 +66,9 @@ __device__ __forceinline__ Prim<double> rt_hd(double (&u)[5], const KParams &p) 
 template <int NVM>
 __device__ __forceinline__ void riemann_mhd(const double (&vl)[NVM], const double (&vr)[NVM],
                                             double (&f)[NVM], const KParams &p, double cmax) {
-#if PIP_RCP
+#if PIP_FAST
+  hlld_flux_fast<NVM>(vl, vr, f, p.gm, p.igm1, cmax);
+#elif PIP_RCP
   hlld_flux_rcp<double, NVM>(vl, vr, f, p.gm, p.igm1, cmax);
 #else
   hlld_flux<double, NVM>(vl, vr, f, p.gm, cmax);
@@ -63,10 +76,24 @@ __device__ __forceinline__ void riemann_mhd(const double (&vl)[NVM], const doubl
 }
 __device__ __forceinline__ void riemann_hd(const double (&vl)[5], const double (&vr)[5],
                                            double (&f)[5], const KParams &p) {
-#if PIP_RCP
+#if PIP_FAST
+  hllc_flux_fast(vl, vr, f, p.gm, p.igm1);
+#elif PIP_RCP
   hllc_flux_rcp<double>(vl, vr, f, p.gm, p.igm1);
 #else
   hllc_flux<double>(vl, vr, f, p.gm);
+#endif
+}
+
+template <int NVM>
+__device__ __forceinline__ void to_prim(const double (&um)[NVM], const double (&uh)[5], double (&vm)[NVM],
+                                        double (&vh)[5], const KParams &p) {
+#if PIP_FAST
+  u2v_mhd_fast<NVM>(um, vm, p.gm, p.ro_lim, p.pr_lim);
+  u2v_hd_fast(uh, vh, p.gm, p.ro_lim, p.pr_lim);
+#else
+  u2v_mhd<double, NVM>(um, vm, p.gm, p.ro_lim, p.pr_lim);
+  u2v_hd<double>(uh, vh, p.gm, p.ro_lim, p.pr_lim);
 #endif
 }
 
@@ -99,6 +126,16 @@ template <int NVM>
 __device__ __forceinline__ void ir_rates(const double (&u)[NVM], const KParams &p, double &gr,
                                          double &gi) {
   const double gm = p.gm;
+#if PIP_FAST
+  const double iro = rcp_(u[0]);
+  double pr = (gm - 1.0) * (u[4] - 0.5 * ((u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) * iro +
+                                          u[5] * u[5] + u[6] * u[6] + u[7] * u[7]));
+  pr = max_(pr, p.pr_lim);
+  const double te = 0.5 * gm * (pr * iro);
+  const double rs = rsqrt_nr(te);
+  gr = p.ir_rec * rs;
+  gi = p.ir_ion * rs * exp(-p.ir_chi * rcp_(te));
+#else
   double pr = (gm - 1.0) * (u[4] - 0.5 * ((u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) / u[0] +
                                           u[5] * u[5] + u[6] * u[6] + u[7] * u[7]));
   pr = fmax(pr, p.pr_lim);
@@ -106,6 +143,7 @@ __device__ __forceinline__ void ir_rates(const double (&u)[NVM], const KParams &
   const double rs = 1.0 / sqrt(te);
   gr = p.ir_rec * rs;
   gi = p.ir_ion * rs * exp(-p.ir_chi / te);
+#endif
 }
 
 constexpr double kPiRef = 3.1415926535897932;  // pi of Parameters.f90:2
@@ -282,10 +320,14 @@ __device__ __forceinline__ void ir_ds(const Prim<double> &qm, const Prim<double>
   ds[3] = gr * qm.de * qm.vz - gi * qh.de * qh.vz;
   const double kin = 0.5 * (gr * qm.de * (qm.vx * qm.vx + qm.vy * qm.vy + qm.vz * qm.vz) -
                             gi * qh.de * (qh.vx * qh.vx + qh.vy * qh.vy + qh.vz * qh.vz));
+#if PIP_FAST
+  ds[4] = kin + ((p.ir_type != 2 ? 0.5 : 1.0) * gr * qm.pr - gi * qh.pr) * p.igm1;
+#else
   if (p.ir_type != 2)
     ds[4] = kin - gi * qh.pr / (gm - 1.0) + 0.5 * gr * qm.pr / (gm - 1.0);
   else
     ds[4] = kin - gi * qh.pr / (gm - 1.0) + gr * qm.pr / (gm - 1.0);
+#endif
 }
 
 // Splits a cell's NV planes into ion and neutral arrays.
@@ -653,8 +695,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         if (p.col_type) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
         if (p.irs) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
       }
-      u2v_mhd<double, NVM>(um, vm, gm, ro_lim, pr_lim);
-      u2v_hd<double>(uh, vh, gm, ro_lim, pr_lim);
+      to_prim<NVM>(um, uh, vm, vh, p);
 #pragma unroll
       for (int n = 0; n < NVM; ++n) sV[n * RR + idx] = vm[n];
 #pragma unroll
@@ -677,8 +718,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       if (p.col_type) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
       if (p.irs) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
     }
-    u2v_mhd<double, NVM>(um, vm, gm, ro_lim, pr_lim);
-    u2v_hd<double>(uh, vh, gm, ro_lim, pr_lim);
+    to_prim<NVM>(um, uh, vm, vh, p);
 #pragma unroll
     for (int n = 0; n < NVM; ++n) sV[n * RR + idx] = vm[n];
 #pragma unroll
@@ -743,12 +783,10 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         // direction 2 swaps (vx,vy) and (bx,by) (set_HLLD_fluxes, HLL_rot.f90:365-383)
         const int src = perm_y ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
         const double *v = sV + src * RR + a;
-        const double v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-        vl[n] = v1 + 0.5 * minmod<double>(v0, v1, v2);
-        vr[n] = v2 - 0.5 * minmod<double>(v1, v2, v3);
+        face_pair(v[-s], v[0], v[s], v[2 * s], vl[n], vr[n]);
       }
-      vl[0] = fmax(vl[0], ro_lim);
-      vr[0] = fmax(vr[0], ro_lim);
+      vl[0] = max_(vl[0], ro_lim);
+      vr[0] = max_(vr[0], ro_lim);
       riemann_mhd<NVM>(vl, vr, fx, p, cmax);
 #pragma unroll
       for (int n = 0; n < NVM; ++n) {
@@ -762,12 +800,10 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       for (int n = 0; n < 5; ++n) {
         const int src = perm_y ? (n == 1 ? 2 : n == 2 ? 1 : n) : n;
         const double *v = sV + (NVM + src) * RR + a;
-        const double v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-        vl[n] = v1 + 0.5 * minmod<double>(v0, v1, v2);
-        vr[n] = v2 - 0.5 * minmod<double>(v1, v2, v3);
+        face_pair(v[-s], v[0], v[s], v[2 * s], vl[n], vr[n]);
       }
-      vl[0] = fmax(vl[0], ro_lim);
-      vr[0] = fmax(vr[0], ro_lim);
+      vl[0] = max_(vl[0], ro_lim);
+      vr[0] = max_(vr[0], ro_lim);
       riemann_hd(vl, vr, fx, p);
 #pragma unroll
       for (int n = 0; n < 5; ++n) {
@@ -823,6 +859,64 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     const double dt_coll = dt * 0.5;                          // set_dt_coll, t_order=2
     double a_m[NVM], a_h[5];  // U0 of the cell
     load_cell<NVM>(U0, q, nc, a_m, a_h);
+    double ac_s = p.ac;       // alpha_c of the stage
+    double S_m[5], S_h[5];
+    Prim<double> qm, qh;      // primitives of the stage state as source_PIP's cq2pv leaves them
+    double gr = 0.0, gion = 0.0;
+    if constexpr (PIP_FAST && !COL) {
+      // The FMA build without per-stage coefficients takes them from the tile (they are
+      // u2v's, the same up to rounding) and forms the exchange from them, so stage 2 does
+      // not read its stage state again; where the density floor acts, u2v's velocity is
+      // another one and the state is converted as the reference does.
+      const int c = (NDIM == 2 ? (tj + kH) * RX : 0) + ti + kH;
+      qm = Prim<double>{sV[c], sV[RR + c], sV[2 * RR + c], sV[3 * RR + c], sV[4 * RR + c]};
+      qh = Prim<double>{sV[NVM * RR + c], sV[(NVM + 1) * RR + c], sV[(NVM + 2) * RR + c],
+                        sV[(NVM + 3) * RR + c], sV[(NVM + 4) * RR + c]};
+      if (!(qm.de > ro_lim && qh.de > ro_lim)) {
+        double s_m[NVM], s_h[5];
+        load_cell<NVM>(STAGE == 1 ? U0 : Us, q, nc, s_m, s_h);
+        qh = rt_hd(s_h, p);
+        qm = rt_mhd<NVM>(s_m, p);
+      }
+      if (p.ir) ir_rates<NVM>(a_m, p, gr, gion);
+      double ds[5];
+      if (p.imp && STAGE == 2) {
+        // exponential form: U0 carries the collision increments of the earlier stages
+        double i0_, i1_;
+        Prim<double> rm = prim_mhd<NVM>(a_m, gm, i0_), rh = prim_hd(a_h, gm, i1_);
+        if (!(above_floors(rm, ro_lim, pr_lim) && above_floors(rh, ro_lim, pr_lim))) {
+          double r_m[NVM], r_h[5];
+#pragma unroll
+          for (int n = 0; n < NVM; ++n) r_m[n] = a_m[n];
+#pragma unroll
+          for (int n = 0; n < 5; ++n) r_h[n] = a_h[n];
+          rh = rt_hd(r_h, p);
+          rm = rt_mhd<NVM>(r_m, p);
+        }
+        collision_prim(rm, rh, p, ac_s, dt_coll, ds);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+          a_h[n] = a_h[n] - dt_coll * ds[n];
+          a_m[n] = a_m[n] + dt_coll * ds[n];
+        }
+      }
+      collision_prim(qm, qh, p, ac_s, dt_coll, ds);
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        if (p.imp) {
+          a_h[n] = a_h[n] - dt_coll * ds[n];
+          a_m[n] = a_m[n] + dt_coll * ds[n];
+        }
+        S_m[n] = p.imp ? 0.0 : ds[n];
+      }
+      if (p.ir) {
+        ir_ds(qm, qh, gr, gion, p, ds);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) S_m[n] = S_m[n] - ds[n];
+      }
+#pragma unroll
+      for (int n = 0; n < 5; ++n) S_h[n] = -S_m[n];
+    } else {
     double s_m[NVM], s_h[5];  // stage state of the cell
     if (STAGE == 1) {
 #pragma unroll
@@ -833,9 +927,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       load_cell<NVM>(Us, q, nc, s_m, s_h);
     }
     // alpha_c of the stage (set_coefficients at the stage start; U0 keeps its energies)
-    double ac_s = p.ac;
     if (COL && p.col_type) ac_s = set_collisional_cell<NVM>(s_m, s_h, p);
-    double gr = 0.0, gion = 0.0;
     if (COL && p.irs) {
       set_ir_cell<NVM>(s_m, s_h, p, gr, gion);  // set_IR of the stage
       if (p.irn) {                              // type 4: nlev_rates_kernel's rates
@@ -872,10 +964,9 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       }
     }
     // source_PIP on the stage state (rewrites it through primitives first)
-    double S_m[5], S_h[5];
     {
-      const Prim<double> qh = rt_hd(s_h, p);
-      const Prim<double> qm = rt_mhd<NVM>(s_m, p);
+      qh = rt_hd(s_h, p);
+      qm = rt_mhd<NVM>(s_m, p);
       double ds[5];
       collision_ds<NVM>(s_m, s_h, qm, qh, p, ac_s, dt_coll, ds);
       if (p.imp) {
@@ -904,9 +995,15 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         if (p.irn && p.ir_type == 0) S_m[4] = S_m[4] - p.nl_ip[q] + 0.0;
       }
     }
+    }
     // time_integral: add_flux_rk (x, then y) and add_source, per species
+#if PIP_FAST
+    const double cx = dt_sub * rcp_(p.dx[gi]);
+    const double cy = NDIM == 2 ? dt_sub * rcp_(p.dy[gj]) : 0.0;
+#else
     const double cx = dt_sub / p.dx[gi];
     const double cy = NDIM == 2 ? dt_sub / p.dy[gj] : 0.0;
+#endif
     const int fxl = tj * (TX + 1) + ti, fyl = tj * TX + ti;
     double n_m[NVM], n_h[5];
 #pragma unroll
@@ -925,6 +1022,34 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 
     // fused cfl rewrites (and the next step's CFL terms)
     const int ep = STAGE == 1 ? 0 : s_epi;  // stage 1 is never followed by a cfl
+#if PIP_FAST
+    if (ep >= 1 && !(COL && p.irl)) {
+      // Away from the floors cq2pv's rewrite is the identity up to rounding, so the state is
+      // left as it is and the second cfl's terms come from the same primitives; where a floor
+      // acts both rewrites are made.
+      double im, ih;
+      Prim<double> em = prim_mhd<NVM>(n_m, gm, im), eh = prim_hd(n_h, gm, ih);
+      if (!(above_floors(em, ro_lim, pr_lim) && above_floors(eh, ro_lim, pr_lim))) {
+        em = rt_mhd<NVM>(n_m, p);
+        eh = rt_hd(n_h, p);
+        if (ep == 2) {
+          em = rt_mhd<NVM>(n_m, p);
+          eh = rt_hd(n_h, p);
+        }
+      }
+      if (ep == 2) {
+        const double gmin = fmin(fmin(p.dx[gi], NDIM == 2 ? p.dy[gj] : p.dy[0]), p.dz0);
+        dtc = cfl_cell_fast(em, eh, n_m[5], n_m[6], n_m[7], gm, p.safety * gmin);
+        rhoc = max_(n_m[0], n_h[0]) * ac_s;
+        if (p.ir) {
+          double g1, g2;
+          ir_rates<NVM>(n_m, p, g1, g2);
+          grc = max_(g1, g2);
+        }
+      }
+    } else
+#endif
+    {
     if (ep >= 1) {
       if (COL && p.irl) {  // the time loop's set_IR before the cfl (main.f90:44-46)
         double g1, g2;
@@ -958,11 +1083,14 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         grc = fmax(g1, g2);
       }
     }
-    bool bad = false;
+    }
+    // non-finite values have an all-ones exponent
+    int top = 0;
 #pragma unroll
-    for (int n = 0; n < NVM; ++n) bad |= !isfinite(n_m[n]);
+    for (int n = 0; n < NVM; ++n) top = max(top, __double2hiint(n_m[n]) & 0x7fffffff);
 #pragma unroll
-    for (int n = 0; n < 5; ++n) bad |= !isfinite(n_h[n]);
+    for (int n = 0; n < 5; ++n) top = max(top, __double2hiint(n_h[n]) & 0x7fffffff);
+    const bool bad = top >= 0x7ff00000;
     if (bad) atomicOr(&ctrl->nan_flag, 1);
     store_cell<NDIM, NVM>(Uo, p, gi, gj, n_m, n_h);
     if (STAGE == 2 && COL && p.col_type) {
@@ -1126,8 +1254,7 @@ __global__ void flux_kernel(const KParams p, const double *__restrict__ U, doubl
     for (int c = 0; c < 4; ++c) {
       double um[NVM], uh[5], vm[NVM], vh[5];
       load_cell<NVM>(U, qa + (c - 1) * s, nc, um, uh);
-      u2v_mhd<double, NVM>(um, vm, gm, ro_lim, pr_lim);
-      u2v_hd<double>(uh, vh, gm, ro_lim, pr_lim);
+      to_prim<NVM>(um, uh, vm, vh, p);
       for (int n = 0; n < NVM; ++n) V[c][n] = vm[n];
       for (int n = 0; n < 5; ++n) V[c][NVM + n] = vh[n];
     }
@@ -1136,11 +1263,10 @@ __global__ void flux_kernel(const KParams p, const double *__restrict__ U, doubl
       double vl[NVM], vr[NVM], fx[NVM];
       for (int n = 0; n < NVM; ++n) {
         const int src = py ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
-        vl[n] = V[1][src] + 0.5 * minmod<double>(V[0][src], V[1][src], V[2][src]);
-        vr[n] = V[2][src] - 0.5 * minmod<double>(V[1][src], V[2][src], V[3][src]);
+        face_pair(V[0][src], V[1][src], V[2][src], V[3][src], vl[n], vr[n]);
       }
-      vl[0] = fmax(vl[0], ro_lim);
-      vr[0] = fmax(vr[0], ro_lim);
+      vl[0] = max_(vl[0], ro_lim);
+      vr[0] = max_(vr[0], ro_lim);
       riemann_mhd<NVM>(vl, vr, fx, p, cmax);
       for (int n = 0; n < NVM; ++n) {
         const int dst = py ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
@@ -1158,11 +1284,10 @@ __global__ void flux_kernel(const KParams p, const double *__restrict__ U, doubl
       double vl[5], vr[5], fx[5];
       for (int n = 0; n < 5; ++n) {
         const int src = NVM + (py ? (n == 1 ? 2 : n == 2 ? 1 : n) : n);
-        vl[n] = V[1][src] + 0.5 * minmod<double>(V[0][src], V[1][src], V[2][src]);
-        vr[n] = V[2][src] - 0.5 * minmod<double>(V[1][src], V[2][src], V[3][src]);
+        face_pair(V[0][src], V[1][src], V[2][src], V[3][src], vl[n], vr[n]);
       }
-      vl[0] = fmax(vl[0], ro_lim);
-      vr[0] = fmax(vr[0], ro_lim);
+      vl[0] = max_(vl[0], ro_lim);
+      vr[0] = max_(vr[0], ro_lim);
       riemann_hd(vl, vr, fx, p);
       for (int n = 0; n < 5; ++n) {
         const int dst = py ? (n == 1 ? 2 : n == 2 ? 1 : n) : n;
@@ -1301,16 +1426,21 @@ static cudaError_t set_stage_attr() {
   cudaError_t e;
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 0>()) != cudaSuccess) return e;
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 1>()) != cudaSuccess) return e;
+#if !PIP_HEAT_ONLY
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 2>()) != cudaSuccess) return e;
-  return set_stage_attr_x<NDIM, NVM, STAGE, 3>();
+  if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 3>()) != cudaSuccess) return e;
+#endif
+  return cudaSuccess;
 }
 
 // Raises the dynamic shared-memory limit of every stage-kernel instance on the current
 // device; called once per context so that graph capture sees launches only.
 static cudaError_t prepare() {
   cudaError_t e;
+#if !PIP_HEAT_ONLY
   if ((e = set_stage_attr<1, 8, 1>()) != cudaSuccess) return e;
   if ((e = set_stage_attr<1, 8, 2>()) != cudaSuccess) return e;
+#endif
   if ((e = set_stage_attr<2, 8, 1>()) != cudaSuccess) return e;
   if ((e = set_stage_attr<2, 8, 2>()) != cudaSuccess) return e;
   if ((e = set_stage_attr<2, 9, 1>()) != cudaSuccess) return e;
@@ -1340,6 +1470,7 @@ static cudaError_t launch_stage_t(const KParams &p, const double *Us, const doub
       stage_kernel<NDIM, NVM, STAGE, 1><<<grid, NT, stage_smem_bytes<NDIM, NVM, 1>(), s>>>(
           p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
       break;
+#if !PIP_HEAT_ONLY
     case 2:
       stage_kernel<NDIM, NVM, STAGE, 2><<<grid, NT, stage_smem_bytes<NDIM, NVM, 2>(), s>>>(
           p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
@@ -1348,6 +1479,10 @@ static cudaError_t launch_stage_t(const KParams &p, const double *Us, const doub
       stage_kernel<NDIM, NVM, STAGE, 3><<<grid, NT, stage_smem_bytes<NDIM, NVM, 3>(), s>>>(
           p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
       break;
+#else
+    default:
+      return cudaErrorInvalidValue;
+#endif
   }
   return cudaGetLastError();
 }
@@ -1355,10 +1490,14 @@ static cudaError_t launch_stage_t(const KParams &p, const double *Us, const doub
 static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
                                 double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                 const CUtensorMap *tm, int rows) {
+#if PIP_HEAT_ONLY
+  if (p.ndim != 2) return cudaErrorInvalidValue;
+#else
   if (p.ndim == 1) {
     return stage == 1 ? launch_stage_t<1, 8, 1>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0)
                       : launch_stage_t<1, 8, 2>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0);
   }
+#endif
   if (p.nvm == 9)
     return stage == 1 ? launch_stage_t<2, 9, 1>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
                       : launch_stage_t<2, 9, 2>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
