@@ -325,6 +325,7 @@ void build_kparams(pip_ctx *c) {
       for (int n = 0; n < pip::kMaxPlanes; ++n) k.symy[s][n] = 1;
     }
   }
+  pip::set_flips(k);
 }
 
 }  // namespace
@@ -398,6 +399,7 @@ int pip::kparams_from_params(const pip_params *p, KParams *k) {
       for (int n = 0; n < pip::kMaxPlanes; ++n) k->symy[s][n] = 1;
     }
   }
+  pip::set_flips(*k);
   return PIP_OK;
 }
 

@@ -327,15 +327,16 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
       for (int n = 0; n < NVM; ++n) bad |= !isfinite(n_m[n]);
 #pragma unroll
       for (int n = 0; n < 5; ++n) bad |= !isfinite(n_h[n]);
+      double u[NV];
 #pragma unroll
       for (int n = 0; n < NV; ++n) {
-        const double u = n < NVM ? n_m[n] : n_h[n - NVM];
-        const float hi = (float)u;
+        u[n] = n < NVM ? n_m[n] : n_h[n - NVM];
+        const float hi = (float)u[n];
         Ohi[gi + n * nc] = hi;
-        if (STAGE == 2) Alo[gi + n * nc] = (float)(u - (double)hi);
+        if (STAGE == 2) Alo[gi + n * nc] = (float)(u[n] - (double)hi);
       }
-      if (mixed::near_boundary<1>(p, gi, 0))
-        mixed::write_ghosts<1>(p, gi, 0, Ohi, STAGE == 2 ? Alo : nullptr, NV);
+      if (near_boundary<1>(p, gi, 0))
+        mixed::write_ghosts<1, NV, STAGE == 2>(p, gi, 0, Ohi, Alo, u);
     }
     __syncthreads();
   }
@@ -417,7 +418,7 @@ __device__ void run_member_2d(const KParams &p, float *Ahi, float *Alo, float *B
   __syncthreads();
   for (long long t = tid; t < (long long)p.nx * p.ny; t += NT) {
     const int gi = p.m0 + (int)(t % p.nx), gj = p.m1 + (int)(t / p.nx);
-    if (mixed::near_boundary<2>(p, gi, gj)) mixed::write_ghosts<2>(p, gi, gj, Ahi, Alo, NV2);
+    if (near_boundary<2>(p, gi, gj)) mixed::copy_ghosts<2, NV2>(p, gi, gj, Ahi, Alo);
   }
   __syncthreads();
   const int ntx = (p.nx + TX2 - 1) / TX2, nty = (p.ny + TY2 - 1) / TY2, ntiles = ntx * nty;
@@ -521,7 +522,7 @@ __device__ __noinline__ void run_member_1d(const KParams &p, float *Ahi, float *
   // the prologue's PIPbnd after its cfl (Initial_rot.f90:152-159)
   __syncthreads();
   for (int i = p.m0 + rank * NT + tid; i < p.ix - p.m0; i += NT * CL)
-    if (mixed::near_boundary<1>(p, i, 0)) mixed::write_ghosts<1>(p, i, 0, Ahi, Alo, NVM + 5);
+    if (near_boundary<1>(p, i, 0)) mixed::copy_ghosts<1, NVM + 5>(p, i, 0, Ahi, Alo);
   member_sync<CL>();
   const int per = (p.nx + CL - 1) / CL;
   const int cb = p.m0 + min(p.nx, rank * per), ce = p.m0 + min(p.nx, (rank + 1) * per);

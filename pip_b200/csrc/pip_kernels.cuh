@@ -87,8 +87,20 @@ struct KParams {
   // boundary maps: ghost layer q of side s (0 lower, 1 upper) copies interior index g?[s][q]
   int gx[2][kMaxMargin], gy[2][kMaxMargin];
   signed char symx[2][kMaxPlanes], symy[2][kMaxPlanes];
+  unsigned flipx[2], flipy[2];   // bit n: the sign table of the face negates plane n
   int typex[2], typey[2];
 };
+
+// The sign tables as bit masks (host; after symx and symy are set).
+inline void set_flips(KParams &k) {
+  for (int s = 0; s < 2; ++s) {
+    k.flipx[s] = k.flipy[s] = 0u;
+    for (int n = 0; n < kMaxPlanes; ++n) {
+      if (k.symx[s][n] < 0) k.flipx[s] |= 1u << n;
+      if (k.symy[s][n] < 0) k.flipy[s] |= 1u << n;
+    }
+  }
+}
 
 // Device-resident loop state of pip_run (main.f90's time, dt and stop flags).
 struct DevCtrl {
@@ -100,7 +112,10 @@ struct DevCtrl {
   unsigned long long red_ip[2];   // set_IR type 4, flag_IR_type 0: max(ion_pot/e_int, 1e-5)
   unsigned long long red_nx[2];   // set_IR type 4: max(dNexcite/dt, 1e-5)
   int last, done, nan_flag, status;
-  unsigned int blocks_done;       // last-block-done counter of the stage-2 kernel
+  // Set by block 0 of stage 1 for stage 2, which does not read what its own block 0 changes
+  // (step, time, done): whether the step is skipped, and the reduction slot of the next dt.
+  int skip, slot;
+  unsigned int blocks_done;       // last-block-done counter of the stage-2 kernel (resi 2)
 };
 
 // Host launchers (one set per arithmetic flavour).

@@ -55,10 +55,13 @@ __device__ __forceinline__ double bitsd(unsigned long long b) {
 }
 
 __device__ __forceinline__ double finalize_dt(const KParams &p, const DevCtrl *c, int slot) {
-  double dt = bitsd(c->red_dt[slot]);
-  double rho = bitsd(c->red_rho[slot]);
+  // both slots are loaded, so that the loads do not wait for the step count
+  const unsigned long long d0 = c->red_dt[0], d1 = c->red_dt[1], r0 = c->red_rho[0], r1 = c->red_rho[1],
+                           g0 = c->red_gr[0], g1 = c->red_gr[1];
+  double dt = bitsd(slot ? d1 : d0);
+  const double rho = bitsd(slot ? r1 : r0);
   dt = fmin(dt, p.col_lim / rho);
-  if (p.ir) dt = fmin(dt, p.ir_lim / fmax(bitsd(c->red_gr[slot]), 1.0e-5));
+  if (p.ir) dt = fmin(dt, p.ir_lim / fmax(bitsd(slot ? g1 : g0), 1.0e-5));
   return dt;
 }
 
@@ -93,8 +96,7 @@ __device__ __forceinline__ void block_reduce_cfl(double dtc, double rho, double 
 
 // One RK stage (see the FP64 stage_kernel for the structure).  Stage 1: Us = A.hi,
 // U0 = A.hi, output B (FP32).  Stage 2: Us = B, U0 = A.hi + A.lo, output A (hi, lo).
-// The parameter block is __grid_constant__: the out-of-line ghost writer takes its address,
-// which would otherwise copy the whole block to every thread's stack.  With use_tma (2D),
+// With use_tma (2D),
 // the tile and its halo of all planes of Us arrive by one TMA load (tmap describes Us).
 template <int NDIM, int NVM, int STAGE>
 __global__ void __launch_bounds__(Tile<NDIM>::NT, NDIM == 2 ? PIP_MIXED_MINB : 4)
@@ -118,8 +120,7 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
   static_assert((NV * RR * sizeof(float)) % sizeof(double) == 0, "Dedner planes alignment");
   __shared__ __align__(8) unsigned long long s_bar;
   __shared__ double s_dt, s_cmax;
-  __shared__ long long s_step;
-  __shared__ int s_exit, s_epi;
+  __shared__ int s_exit, s_epi, s_slot;
 
   const int tid = threadIdx.x;
   // tile row: every row (rows 0), the first and the last (1), the rows between them (2)
@@ -127,68 +128,92 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
   const int by = NDIM == 1 || rows == 0 ? (int)blockIdx.y
                  : rows == 1 ? (blockIdx.y == 0 ? 0 : nby - 1) : (int)blockIdx.y + 1;
   const bool block0 = blockIdx.x == 0 && by == 0;
+  const int i0 = p.m0 + blockIdx.x * TX;
+  const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
+  // (the TMA writes shared memory only at 128-byte aligned destinations)
+  const bool staged = NDIM == 2 && use_tma && (tma_smem_addr(sV) & 127u) == 0;
+  if (tid == 0 && staged) tma_bar_init(&s_bar);
+  // launched as a programmatic dependent of the previous kernel (see the FP64 stage_kernel)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
-    int ex = STAGE == 1 ? (ctrl->done || ctrl->nan_flag) : ctrl->done;
+    if (staged) {
+      // the raw planes by one TMA load into sV (cells outside the array read as zero), in
+      // flight while the control block is read; the tile step forms the primitives in place
+      tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(float)));
+      tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
+    }
     double dt, cmax;
-    if (STAGE == 1 && dt_mode == 1) {
-      dt = finalize_dt(p, ctrl, (int)(ctrl->step & 1));
-      cmax = p.sg_all / dt;
-    } else {
+    if (STAGE == 1) {
+      const int done = ctrl->done, nan = ctrl->nan_flag;
+      const long long st = ctrl->step;
       dt = ctrl->dt;
       cmax = ctrl->cmax;
+      if (dt_mode == 1) {
+        dt = finalize_dt(p, ctrl, (int)(st & 1));
+        cmax = p.sg_all / dt;
+      }
+      s_exit = done || nan;
+      s_epi = epi;
+      s_slot = 0;
+    } else {
+      const int skip = ctrl->skip, slot = ctrl->slot, last = ctrl->last, status = ctrl->status;
+      dt = ctrl->dt;
+      cmax = ctrl->cmax;
+      s_exit = skip || status == 5;
+      s_epi = epi < 0 ? (last ? 1 : 2) : epi;
+      s_slot = slot;
     }
     s_dt = dt;
     s_cmax = cmax;
-    s_step = ctrl->step;
-    s_exit = ex;
-    s_epi = (STAGE == 2 && epi < 0) ? (ctrl->last ? 1 : 2) : epi;
   }
   __syncthreads();
   if (s_exit) {
     if (STAGE == 1 && block0 && tid == 0) {
       if (ctrl->nan_flag && ctrl->status == 0) ctrl->status = 3;
       ctrl->done = 1;
+      ctrl->skip = 1;
     }
+    if (staged) tma_bar_wait(&s_bar, kTmaWaitLimit);   // no copy in flight when the CTA leaves
     return;
   }
   const double dt = s_dt;
-  if (STAGE == 1 && dt_mode == 1 && block0 && tid == 0) {
-    const long long st = ctrl->step;
-    ctrl->dt = dt;
-    ctrl->cmax = s_cmax;
-    const double tn = ctrl->time + dt;
-    ctrl->time_next = tn;
-    ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
-                  (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
-    const int ns = (int)((st + 1) & 1);
-    ctrl->red_dt[ns] = dbits(10.0);
-    ctrl->red_rho[ns] = 0ull;
-    ctrl->red_gr[ns] = 0ull;
+  if (STAGE == 1 && block0 && tid == 0) {
+    ctrl->skip = 0;
+    if (dt_mode == 1) {
+      const long long st = ctrl->step;
+      ctrl->dt = dt;
+      ctrl->cmax = s_cmax;
+      const double tn = ctrl->time + dt;
+      ctrl->time_next = tn;
+      ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
+                    (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
+      const int ns = (int)((st + 1) & 1);
+      ctrl->slot = ns;
+      ctrl->red_dt[ns] = dbits(10.0);
+      ctrl->red_rho[ns] = 0ull;
+      ctrl->red_gr[ns] = 0ull;
+    }
   }
-  const int i0 = p.m0 + blockIdx.x * TX;
-  const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
+  if (STAGE == 2 && dt_mode == 1 && block0 && tid == 0) {
+    // end of step; no block of stage 2 reads what changes here
+    ctrl->time = ctrl->time_next;
+    ctrl->step = ctrl->step + 1;
+    if (ctrl->last) ctrl->done = 1;
+    if (dt <= 1.0e-12) {
+      ctrl->done = 1;
+      if (ctrl->status == 0) ctrl->status = 4;
+    }
+  }
 
   // ---- 1.-3. the tile (primitives, face fluxes, source and update)
-  // (the TMA writes shared memory only at 128-byte aligned destinations)
-  bool staged = false;
-  if (NDIM == 2 && use_tma && (tma_smem_addr(sV) & 127u) == 0) {
-    // the raw planes by one TMA load into sV (cells outside the array read as zero); the
-    // tile step forms the primitives in place
-    if (tid == 0) {
-      tma_bar_init(&s_bar);
-      tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(float)));
-      tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
-    }
-    __syncthreads();
-    if (!tma_bar_wait(&s_bar, kTmaWaitLimit)) {
-      // the tile did not arrive: flag the stage (the run stops with PIP_ERR_ITER; this
-      // tile's results are void) and let the copy land (bounded) before going on, so that
-      // no copy is in flight when the CTA's shared memory is released
-      atomicCAS(&ctrl->status, 0, 5);
-      ctrl->done = 1;
-      tma_bar_wait(&s_bar, kTmaWaitLimit);
-    }
-    staged = true;
+  if (staged && !tma_bar_wait(&s_bar, kTmaWaitLimit)) {
+    // the tile did not arrive: flag the stage (the run stops with PIP_ERR_ITER; this
+    // tile's results are void) and let the copy land (bounded) before going on, so that
+    // no copy is in flight when the CTA's shared memory is released
+    atomicCAS(&ctrl->status, 0, 5);
+    ctrl->done = 1;
+    tma_bar_wait(&s_bar, kTmaWaitLimit);
   }
   double dtc = 10.0, rhoc = 0.0, grc = 0.0;
   bool bad = false;
@@ -196,25 +221,7 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
                                               s_epi, staged, sV, sD6, sD9, sFx, sFy, dtc, rhoc,
                                               grc, bad);
   if (bad) atomicOr(&ctrl->nan_flag, 1);
-  if (STAGE == 2 && s_epi == 2) block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, (int)((s_step + 1) & 1));
-  if (STAGE == 2 && dt_mode == 1) {
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      const unsigned int nb = gridDim.x * nby;     // every tile of the stage's launches
-      if (atomicAdd(&ctrl->blocks_done, 1u) == nb - 1) {
-        __threadfence();
-        ctrl->blocks_done = 0u;
-        ctrl->time = ctrl->time_next;
-        ctrl->step = s_step + 1;
-        if (ctrl->last) ctrl->done = 1;
-        if (dt <= 1.0e-12) {
-          ctrl->done = 1;
-          if (ctrl->status == 0) ctrl->status = 4;
-        }
-      }
-    }
-  }
+  if (STAGE == 2 && s_epi == 2) block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, s_slot);
 }
 
 // cfl over every cell for the mixed state: floors (in FP64 on hi+lo) and FP32 CFL terms.
@@ -308,12 +315,21 @@ static cudaError_t launch_t(const KParams &p, const float *Us, const float *U0hi
   if (NDIM == 1) rows = 0;
   const int gy = rows == 0 ? nby : rows == 1 ? (nby < 2 ? nby : 2) : nby - 2;
   if (gy <= 0) return cudaSuccess;   // no rows between the first and the last
-  dim3 grid((p.nx + TX - 1) / TX, gy);
   CUtensorMap none;
   std::memset(&none, 0, sizeof none);
-  stage_kernel<NDIM, NVM, STAGE><<<grid, NT, smem_bytes<NDIM, NVM>(), s>>>(
-      p, Us, U0hi, U0lo, Ohi, Olo, ctrl, dt_mode, epi, tm ? *tm : none, tm ? 1 : 0, rows);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((p.nx + TX - 1) / TX, gy);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem_bytes<NDIM, NVM>();
+  cfg.stream = s;
+  // a programmatic dependent of the previous kernel (not the rows of a split stage)
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = rows == 0 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, stage_kernel<NDIM, NVM, STAGE>, p, Us, U0hi, U0lo, Ohi, Olo, ctrl,
+                            dt_mode, epi, tm ? *tm : none, tm ? 1 : 0, rows);
 }
 
 static int grid_for(long long n, int threads) {

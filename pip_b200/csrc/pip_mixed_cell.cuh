@@ -3,6 +3,7 @@
 // kernels and the batched ensemble so that both compute identical cell updates.
 #pragma once
 
+#include "pip_ghosts.cuh"
 #include "pip_kernels.cuh"
 #include "pip_physics.cuh"
 
@@ -136,59 +137,39 @@ __device__ __forceinline__ void ir_ds(const Prim<double> &qm, const Prim<double>
     ds[4] = kin - gi * qh.pr / (gm - 1.0) + gr * qm.pr / (gm - 1.0);
 }
 
-// Ghost images of one updated cell (PIPbnd after the stage, x faces then y faces, so a
-// corner ghost carries both sign flips).  Only cells within 2*margin of a boundary can be
-// a ghost source; the caller tests that first.  The values are re-read from the planes the
-// same thread has just written.
-template <int NDIM>
-__device__ __forceinline__ bool near_boundary(const KParams &p, int gi, int gj) {
-  return gi < 2 * p.m0 || gi >= p.ix - 2 * p.m0 ||
-         (NDIM == 2 && (gj < 2 * p.m1 || gj >= p.jx - 2 * p.m1));
+// Ghost images of a cell whose NP FP64 values u are stored as hi (and, with PAIR, lo) planes:
+// hi = (float)u, lo = (float)(u - hi), with the faces' sign flips.
+template <int NDIM, int NP, bool PAIR>
+__device__ __forceinline__ void write_ghosts(const KParams &p, int gi, int gj, float *hi, float *lo,
+                                             const double (&u)[NP]) {
+  const long long nc = p.nc;
+  ghost_images<NDIM>(p, gi, gj, [&](long long t, unsigned flips) {
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+      const float h = (float)u[n];
+      hi[t + n * nc] = flipped(h, flips, n);
+      if (PAIR) lo[t + n * nc] = flipped((float)(u[n] - (double)h), flips, n);
+    }
+  });
 }
 
-template <int NDIM>
-__device__ __noinline__ void write_ghosts(const KParams &p, int gi, int gj, float *hi, float *lo,
-                                          int nplanes) {
-  const long long nc = p.nc;
-  const long long q = (long long)gj * p.ix + gi;
-  int tx[2 * kMaxMargin], sx[2 * kMaxMargin], ntx = 0;
-  int ty[2 * kMaxMargin], sy[2 * kMaxMargin], nty = 0;
-  for (int s = 0; s < 2; ++s)
-    for (int l = 0; l < p.m0; ++l)
-      if (p.gx[s][l] == gi) {
-        tx[ntx] = s == 0 ? l : p.ix - p.m0 + l;
-        sx[ntx++] = s;
-      }
-  if (NDIM == 2)
-    for (int s = 0; s < 2; ++s)
-      for (int l = 0; l < p.m1; ++l)
-        if (p.gy[s][l] == gj) {
-          ty[nty] = s == 0 ? l : p.jx - p.m1 + l;
-          sy[nty++] = s;
-        }
-#pragma unroll 1
-  for (int n = 0; n < nplanes; ++n) {
-    const float h = hi[q + n * nc];
-    const float w = lo ? lo[q + n * nc] : 0.0f;
-    for (int a = 0; a < ntx; ++a) {
-      const float g = (float)p.symx[sx[a]][n];
-      const long long t = (long long)gj * p.ix + tx[a];
-      hi[t + n * nc] = g * h;
-      if (lo) lo[t + n * nc] = g * w;
-      for (int b = 0; b < nty; ++b) {
-        const float g2 = (float)p.symy[sy[b]][n];
-        const long long c = (long long)ty[b] * p.ix + tx[a];
-        hi[c + n * nc] = g2 * (g * h);
-        if (lo) lo[c + n * nc] = g2 * (g * w);
-      }
-    }
-    for (int b = 0; b < nty; ++b) {
-      const float g2 = (float)p.symy[sy[b]][n];
-      const long long t = (long long)ty[b] * p.ix + gi;
-      hi[t + n * nc] = g2 * h;
-      if (lo) lo[t + n * nc] = g2 * w;
-    }
+// The same for a cell already stored in hi and lo.
+template <int NDIM, int NP>
+__device__ __forceinline__ void copy_ghosts(const KParams &p, int gi, int gj, float *hi, float *lo) {
+  const long long nc = p.nc, q = (long long)gj * p.ix + gi;
+  float h[NP], w[NP];
+#pragma unroll
+  for (int n = 0; n < NP; ++n) {
+    h[n] = hi[q + n * nc];
+    w[n] = lo[q + n * nc];
   }
+  ghost_images<NDIM>(p, gi, gj, [&](long long t, unsigned flips) {
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+      hi[t + n * nc] = flipped(h[n], flips, n);
+      lo[t + n * nc] = flipped(w[n], flips, n);
+    }
+  });
 }
 
 }  // namespace mixed

@@ -288,14 +288,16 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
     for (int n = 0; n < NVM; ++n) bad |= !isfinite(n_m[n]);
 #pragma unroll
     for (int n = 0; n < 5; ++n) bad |= !isfinite(n_h[n]);
+    double u[NV];
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
-      const double u = n < NVM ? n_m[n] : n_h[n - NVM];
-      const float hi = (float)u;
+      u[n] = n < NVM ? n_m[n] : n_h[n - NVM];
+      const float hi = (float)u[n];
       Ohi[q + n * nc] = hi;
-      if (STAGE == 2) Olo[q + n * nc] = (float)(u - (double)hi);
+      if (STAGE == 2) Olo[q + n * nc] = (float)(u[n] - (double)hi);
     }
-    if (near_boundary<NDIM>(p, gi, gj)) write_ghosts<NDIM>(p, gi, gj, Ohi, STAGE == 2 ? Olo : nullptr, NV);
+    if (near_boundary<NDIM>(p, gi, gj))
+      write_ghosts<NDIM, NV, STAGE == 2>(p, gi, gj, Ohi, Olo, u);
   }
 }
 

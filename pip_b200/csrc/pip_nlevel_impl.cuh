@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(128) nlev_update_kernel(const __grid_constant_
     o[5] = U[q];
 #pragma unroll
     for (int m = 0; m < 6; ++m) p.nl_nex2[q + m * nc] = o[m];
-    if (near_boundary<NDIM>(p, i, j)) write_ghosts<NDIM>(p, i, j, p.nl_nex2, 6, true);
+    if (near_boundary<NDIM>(p, i, j)) write_ghosts<NDIM, 6, false>(p, i, j, p.nl_nex2, o);
   }
 }
 #undef PIP_NL_GT

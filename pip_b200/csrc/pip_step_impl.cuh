@@ -16,6 +16,7 @@
 #include <cstring>
 
 #include "pip_fp64_forms.cuh"
+#include "pip_ghosts.cuh"
 #include "pip_kernels.cuh"
 #include "pip_physics.cuh"
 #include "pip_tma.cuh"
@@ -30,20 +31,30 @@ namespace PIP_FLAVOUR {
 
 constexpr int kH = 2;  // stencil half-width of minmod MUSCL
 
-template <int NDIM> struct Tile;
-// 2D tile (compile-time tuning constants; 32x7 cells: 33x7 x faces + 32x8 y faces = 487
-// faces = two rounds of 256 threads).
+// Tiles.  S = 0, for grids that fill the GPU: 32x7 cells in 2D (33x7 x faces + 32x8 y faces =
+// 487 faces = two rounds of 256 threads), 128 cells in 1D; a thread computes a face of both
+// species.  S = 1, for small grids, whose stages last as long as one tile's chain of dependent
+// operations: 8x4 cells (36 + 40 faces) or 31 cells (32 faces), the species' conversions and
+// faces on separate warps, one round each, so that more SMs share the grid and no thread
+// runs two solvers.  NI: threads of the ions' faces (S = 1; as many for the neutrals').
+template <int NDIM, int S> struct Tile;
 #ifndef PIP_FP64_TX
 #define PIP_FP64_TX 32
 #endif
 #ifndef PIP_FP64_TY
 #define PIP_FP64_TY 7
 #endif
-template <> struct Tile<2> {
-  static constexpr int TX = PIP_FP64_TX, TY = PIP_FP64_TY, NT = (TX * TY + 255) / 256 * 256;
+template <> struct Tile<2, 0> {
+  static constexpr int TX = PIP_FP64_TX, TY = PIP_FP64_TY, NT = 256, MINB = 2, NI = NT;
 };
-template <> struct Tile<1> {
-  static constexpr int TX = 128, TY = 1, NT = 128;
+template <> struct Tile<1, 0> {
+  static constexpr int TX = 128, TY = 1, NT = 128, MINB = 4, NI = NT;
+};
+template <> struct Tile<2, 1> {
+  static constexpr int TX = 8, TY = 4, NT = 192, MINB = 2, NI = 96;
+};
+template <> struct Tile<1, 1> {
+  static constexpr int TX = 31, TY = 1, NT = 64, MINB = 4, NI = 32;
 };
 
 // Conversions and Riemann solvers of this flavour: the literal reference expressions
@@ -86,14 +97,18 @@ __device__ __forceinline__ void riemann_hd(const double (&vl)[5], const double (
 }
 
 template <int NVM>
-__device__ __forceinline__ void to_prim(const double (&um)[NVM], const double (&uh)[5], double (&vm)[NVM],
-                                        double (&vh)[5], const KParams &p) {
+__device__ __forceinline__ void to_prim_mhd(const double (&u)[NVM], double (&v)[NVM], const KParams &p) {
 #if PIP_FAST
-  u2v_mhd_fast<NVM>(um, vm, p.gm, p.ro_lim, p.pr_lim);
-  u2v_hd_fast(uh, vh, p.gm, p.ro_lim, p.pr_lim);
+  u2v_mhd_fast<NVM>(u, v, p.gm, p.ro_lim, p.pr_lim);
 #else
-  u2v_mhd<double, NVM>(um, vm, p.gm, p.ro_lim, p.pr_lim);
-  u2v_hd<double>(uh, vh, p.gm, p.ro_lim, p.pr_lim);
+  u2v_mhd<double, NVM>(u, v, p.gm, p.ro_lim, p.pr_lim);
+#endif
+}
+__device__ __forceinline__ void to_prim_hd(const double (&u)[5], double (&v)[5], const KParams &p) {
+#if PIP_FAST
+  u2v_hd_fast(u, v, p.gm, p.ro_lim, p.pr_lim);
+#else
+  u2v_hd<double>(u, v, p.gm, p.ro_lim, p.pr_lim);
 #endif
 }
 
@@ -107,10 +122,13 @@ __device__ __forceinline__ double bitsd(unsigned long long b) {
 // dt of the step from the reduced CFL terms (cfl, Scheme_rot.f90:183-213): the minimum
 // CFL candidate (seeded with cfl_mhd's 10.0), cfl_pn_col and cfl_pip_ir.
 __device__ __forceinline__ double finalize_dt(const KParams &p, const DevCtrl *c, int slot) {
-  double dt = bitsd(c->red_dt[slot]);
-  double rho = bitsd(c->red_rho[slot]);
+  // both slots are loaded, so that the loads do not wait for the step count
+  const unsigned long long d0 = c->red_dt[0], d1 = c->red_dt[1], r0 = c->red_rho[0], r1 = c->red_rho[1],
+                           g0 = c->red_gr[0], g1 = c->red_gr[1];
+  double dt = bitsd(slot ? d1 : d0);
+  double rho = bitsd(slot ? r1 : r0);
   dt = fmin(dt, p.col_lim / rho);
-  if (p.ir) dt = fmin(dt, p.ir_lim / fmax(bitsd(c->red_gr[slot]), 1.0e-5));
+  if (p.ir) dt = fmin(dt, p.ir_lim / fmax(bitsd(slot ? g1 : g0), 1.0e-5));
   if (p.irn) {
     // cfl_pip_ir's ion_pot term (flag_IR_type 0) and cfl_pip_ir_nexcite; the slots hold
     // the maxima already raised to 1e-5
@@ -340,53 +358,16 @@ __device__ __forceinline__ void load_cell(const double *__restrict__ U, long lon
   for (int n = 0; n < 5; ++n) uh[n] = U[q + (NVM + n) * nc];
 }
 
-// Ghost images of one updated cell (PIPbnd after the stage: x faces first, then y faces,
-// Boundary_rot.f90:54-125 order, so a corner ghost carries both sign flips).  Only cells
-// within 2*margin of a boundary can be a ghost source; the values are re-read from the
-// planes the same thread has just written.
-template <int NDIM>
-__device__ __forceinline__ bool near_boundary(const KParams &p, int gi, int gj) {
-  return gi < 2 * p.m0 || gi >= p.ix - 2 * p.m0 ||
-         (NDIM == 2 && (gj < 2 * p.m1 || gj >= p.jx - 2 * p.m1));
-}
-
-template <int NDIM>
-__device__ __forceinline__ void write_ghosts(const KParams &p, int gi, int gj, double *U, int nplanes,
-                                             bool unsigned_plane = false) {
+// The NP plane values v of cell (gi, gj) into its ghost images, with the sign tables of the
+// faces (SIGNED) or without.
+template <int NDIM, int NP, bool SIGNED>
+__device__ __forceinline__ void write_ghosts(const KParams &p, int gi, int gj, double *U,
+                                             const double (&v)[NP]) {
   const long long nc = p.nc;
-  const long long q = (long long)gj * p.ix + gi;
-  int tx[2 * kMaxMargin], sx[2 * kMaxMargin], ntx = 0;
-  int ty[2 * kMaxMargin], sy[2 * kMaxMargin], nty = 0;
-  for (int s = 0; s < 2; ++s)
-    for (int l = 0; l < p.m0; ++l)
-      if (p.gx[s][l] == gi) {
-        tx[ntx] = s == 0 ? l : p.ix - p.m0 + l;
-        sx[ntx++] = s;
-      }
-  if (NDIM == 2)
-    for (int s = 0; s < 2; ++s)
-      for (int l = 0; l < p.m1; ++l)
-        if (p.gy[s][l] == gj) {
-          ty[nty] = s == 0 ? l : p.jx - p.m1 + l;
-          sy[nty++] = s;
-        }
-#pragma unroll 1
-  for (int n = 0; n < nplanes; ++n) {
-    const double v = U[q + n * nc];
-    for (int a = 0; a < ntx; ++a) {
-      if (unsigned_plane) {
-        U[(long long)gj * p.ix + tx[a] + n * nc] = v;
-        for (int b = 0; b < nty; ++b) U[(long long)ty[b] * p.ix + tx[a] + n * nc] = v;
-        continue;
-      }
-      const double g = (double)p.symx[sx[a]][n];
-      U[(long long)gj * p.ix + tx[a] + n * nc] = g * v;
-      for (int b = 0; b < nty; ++b)
-        U[(long long)ty[b] * p.ix + tx[a] + n * nc] = (double)p.symy[sy[b]][n] * (g * v);
-    }
-    for (int b = 0; b < nty; ++b)
-      U[(long long)ty[b] * p.ix + gi + n * nc] = unsigned_plane ? v : (double)p.symy[sy[b]][n] * v;
-  }
+  ghost_images<NDIM>(p, gi, gj, [&](long long t, unsigned flips) {
+#pragma unroll
+    for (int n = 0; n < NP; ++n) U[t + n * nc] = SIGNED ? flipped(v[n], flips, n) : v[n];
+  });
 }
 
 // Writes a cell and its ghost images.
@@ -395,11 +376,14 @@ __device__ __forceinline__ void store_cell(double *U, const KParams &p, int gi, 
                                            const double (&um)[NVM], const double (&uh)[5]) {
   const long long nc = p.nc;
   const long long q = (long long)gj * p.ix + gi;
+  double v[NVM + 5];
 #pragma unroll
-  for (int n = 0; n < NVM; ++n) U[q + n * nc] = um[n];
+  for (int n = 0; n < NVM; ++n) v[n] = um[n];
 #pragma unroll
-  for (int n = 0; n < 5; ++n) U[q + (NVM + n) * nc] = uh[n];
-  if (near_boundary<NDIM>(p, gi, gj)) write_ghosts<NDIM>(p, gi, gj, U, NVM + 5);
+  for (int n = 0; n < 5; ++n) v[NVM + n] = uh[n];
+#pragma unroll
+  for (int n = 0; n < NVM + 5; ++n) U[q + n * nc] = v[n];
+  if (near_boundary<NDIM>(p, gi, gj)) write_ghosts<NDIM, NVM + 5, true>(p, gi, gj, U, v);
 }
 
 // Block-wide min/max into the reduction slots (one atomic per block).
@@ -575,12 +559,18 @@ __device__ __forceinline__ void block_min_to(double v, unsigned long long *dst) 
   }
 }
 
-template <int NDIM, int NVM, int STAGE, int X>
-__global__ void __launch_bounds__(Tile<NDIM>::NT, NDIM == 2 ? 2 : 4)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <int NDIM, int NVM, int STAGE, int X, int S>
+__global__ void __launch_bounds__(Tile<NDIM, S>::NT, Tile<NDIM, S>::MINB)
 stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, const double *U0,
              double *Uo, DevCtrl *ctrl, int dt_mode, int epi,
              const __grid_constant__ CUtensorMap tmap, int use_tma, int rows) {
-  constexpr int TX = Tile<NDIM>::TX, TY = Tile<NDIM>::TY, NT = Tile<NDIM>::NT;
+  constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = Tile<NDIM, S>::NT;
+  constexpr int NI = Tile<NDIM, S>::NI;
   constexpr int NV = NVM + 5;
   constexpr int RX = TX + 2 * kH, RY = NDIM == 2 ? TY + 2 * kH : 1, RR = RX * RY;
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
@@ -592,8 +582,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   constexpr bool COL = (X & 1) != 0, RES = (X & 2) != 0;
   double *sE = sFy + NV * NFY;  // RES only: E of the tile's cells and one ring
   __shared__ double s_dt, s_cmax;
-  __shared__ long long s_step;
-  __shared__ int s_exit, s_epi;
+  __shared__ int s_exit, s_epi, s_slot;
   __shared__ __align__(8) unsigned long long s_bar;
 
   const int tid = threadIdx.x;
@@ -603,52 +592,87 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   const int by = NDIM == 1 || rows == 0 ? (int)blockIdx.y
                  : rows == 1 ? (blockIdx.y == 0 ? 0 : nby - 1) : (int)blockIdx.y + 1;
   const bool block0 = blockIdx.x == 0 && by == 0;
+  const int i0 = p.m0 + blockIdx.x * TX;
+  const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
+  const bool staged = NDIM == 2 && use_tma && (tma_smem_addr(sV) & 127u) == 0;
+  if (tid == 0 && staged) tma_bar_init(&s_bar);
+  // Launched as a programmatic dependent of the previous kernel on the stream: it may start
+  // while that one finishes, and reads nothing that one wrote before this wait.
+  pdl_wait();
+  pdl_launch_dependents();
   if (tid == 0) {
-    int ex = 0;
-    if (STAGE == 1) {
-      if (ctrl->done || ctrl->nan_flag) ex = 1;
-    } else {
-      if (ctrl->done) ex = 1;
+    if (staged) {
+      // all planes of the tile and its halo by one TMA load into sV (cells outside the array
+      // read as zero), in flight while the control block is read
+      tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
+      tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
     }
+    // the control block by independent loads (one round trip), then dt
     double dt, cmax;
-    if (STAGE == 1 && dt_mode == 1) {
+    if (STAGE == 1) {
+      const int done = ctrl->done, nan = ctrl->nan_flag;
       const long long st = ctrl->step;
-      dt = finalize_dt(p, ctrl, (int)(st & 1));
-      cmax = p.sg_all / dt;
-    } else {
       dt = ctrl->dt;
       cmax = ctrl->cmax;
+      if (dt_mode == 1) {
+        dt = finalize_dt(p, ctrl, (int)(st & 1));
+        cmax = p.sg_all / dt;
+      }
+      s_exit = done || nan;
+      s_epi = epi;
+      s_slot = 0;
+    } else {
+      const int skip = ctrl->skip, slot = ctrl->slot, last = ctrl->last, status = ctrl->status;
+      dt = ctrl->dt;
+      cmax = ctrl->cmax;
+      s_exit = skip || status == 5;    // 5: a tile of stage 1 did not arrive
+      s_epi = epi < 0 ? (last ? 1 : 2) : epi;
+      s_slot = slot;
     }
     s_dt = dt;
     s_cmax = cmax;
-    s_step = ctrl->step;
-    s_exit = ex;
-    s_epi = (STAGE == 2 && epi < 0) ? (ctrl->last ? 1 : 2) : epi;
   }
   __syncthreads();
   if (s_exit) {
     if (STAGE == 1 && block0 && tid == 0) {
       if (ctrl->nan_flag && ctrl->status == 0) ctrl->status = 3;  // PIP_ERR_NAN
       ctrl->done = 1;
+      ctrl->skip = 1;
     }
+    if (staged) tma_bar_wait(&s_bar, kTmaWaitLimit);   // no copy in flight when the CTA leaves
     return;
   }
   const double dt = s_dt, cmax = s_cmax;
-  if (STAGE == 1 && dt_mode == 1 && block0 && tid == 0) {
-    // loop bookkeeping of main.f90:31,58 for this step
-    const long long st = ctrl->step;
-    ctrl->dt = dt;
-    ctrl->cmax = cmax;
-    const double tn = ctrl->time + dt;
-    ctrl->time_next = tn;
-    ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
-                  (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
-    const int ns = (int)((st + 1) & 1);
-    ctrl->red_dt[ns] = dbits(fmin(10.0, p.resi_dt));  // cfl_mhd's start, cfl_resi's bound
-    ctrl->red_rho[ns] = 0ull;
-    ctrl->red_gr[ns] = 0ull;
-    ctrl->red_ip[ns] = 0ull;
-    ctrl->red_nx[ns] = 0ull;
+  if (STAGE == 1 && block0 && tid == 0) {
+    ctrl->skip = 0;
+    if (dt_mode == 1) {
+      // loop bookkeeping of main.f90:31,58 for this step (no block of stage 1 reads these)
+      const long long st = ctrl->step;
+      ctrl->dt = dt;
+      ctrl->cmax = cmax;
+      const double tn = ctrl->time + dt;
+      ctrl->time_next = tn;
+      ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
+                    (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
+      const int ns = (int)((st + 1) & 1);
+      ctrl->slot = ns;
+      ctrl->red_dt[ns] = dbits(fmin(10.0, p.resi_dt));  // cfl_mhd's start, cfl_resi's bound
+      ctrl->red_rho[ns] = 0ull;
+      ctrl->red_gr[ns] = 0ull;
+      ctrl->red_ip[ns] = 0ull;
+      ctrl->red_nx[ns] = 0ull;
+    }
+  }
+  if (STAGE == 2 && dt_mode == 1 && !(RES && p.resi == 2) && block0 && tid == 0) {
+    // end of step: time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636); no
+    // block of stage 2 reads what changes here
+    ctrl->time = ctrl->time_next;
+    ctrl->step = ctrl->step + 1;
+    if (ctrl->last) ctrl->done = 1;
+    if (dt <= 1.0e-12) {
+      ctrl->done = 1;
+      if (ctrl->status == 0) ctrl->status = 4;  // PIP_ERR_DT
+    }
   }
 
   if (STAGE == 1 && RES && p.resi == 2 && block0 && tid == 0) {
@@ -658,59 +682,30 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   }
 
   const double gm = p.gm, ro_lim = p.ro_lim, pr_lim = p.pr_lim;
-  const int i0 = p.m0 + blockIdx.x * TX;
-  const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
   const long long nc = p.nc;
 
   // ---- 1. stage state of the tile and its halo -> primitives in shared memory
-  if (NDIM == 2 && use_tma && (tma_smem_addr(sV) & 127u) == 0) {
-    // all planes of the tile and its halo by one TMA load into sV (cells outside the array
-    // read as zero), then the primitives in place, each thread on its own cells
-    if (tid == 0) {
-      tma_bar_init(&s_bar);
-      tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
-      tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
-    }
-    __syncthreads();
-    if (!tma_bar_wait(&s_bar, kTmaWaitLimit)) {
-      // the tile did not arrive: flag the stage (the run stops with PIP_ERR_ITER; this
-      // tile's results are void) and let the copy land (bounded) before going on, so that
-      // no copy is in flight when the CTA's shared memory is released
-      atomicCAS(&ctrl->status, 0, 5);
-      ctrl->done = 1;
-      tma_bar_wait(&s_bar, kTmaWaitLimit);
-    }
-    for (int idx = tid; idx < RR; idx += NT) {
-      const int ri = idx % RX, rj = idx / RX;
-      if (!RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH)) continue;
-      const int gi = i0 - kH + ri, gj = j0 - kH + rj;
-      if (gi >= p.ix || gj >= p.jx) continue;
-      double um[NVM], uh[5], vm[NVM], vh[5];
-#pragma unroll
-      for (int n = 0; n < NVM; ++n) um[n] = sV[n * RR + idx];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) uh[n] = sV[(NVM + n) * RR + idx];
-      if (COL) {
-        double te_m, te_h, rm, rh;
-        if (p.col_type) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
-        if (p.irs) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
-      }
-      to_prim<NVM>(um, uh, vm, vh, p);
-#pragma unroll
-      for (int n = 0; n < NVM; ++n) sV[n * RR + idx] = vm[n];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) sV[(NVM + n) * RR + idx] = vh[n];
-    }
-  } else
-  for (int idx = tid; idx < RR; idx += NT) {
-    const int ri = idx % RX, rj = idx / RX;
-    // the corners only for the curl of B next to the tile's corner faces (resistivity)
-    if (NDIM == 2 && !RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH))
-      continue;
-    const int gi = i0 - kH + ri, gj = NDIM == 2 ? j0 - kH + rj : 0;
-    if (gi >= p.ix || gj >= p.jx) continue;
+  // Each cell's conversion is one thread's (both species); with S = 1 and no energy rewrite
+  // a unit is one species of a cell.  The TMA's tile is converted in place.
+  if (staged && !tma_bar_wait(&s_bar, kTmaWaitLimit)) {
+    // the tile did not arrive: flag the stage (the run stops with PIP_ERR_ITER; this
+    // tile's results are void) and let the copy land (bounded) before going on, so that
+    // no copy is in flight when the CTA's shared memory is released
+    atomicCAS(&ctrl->status, 0, 5);
+    ctrl->done = 1;
+    tma_bar_wait(&s_bar, kTmaWaitLimit);
+  }
+  constexpr bool SPLITP = S == 1 && !COL;
+  auto convert = [&](const double *src, long long sp, int idx, bool ions, bool neutrals) {
     double um[NVM], uh[5], vm[NVM], vh[5];
-    load_cell<NVM>(Us, (long long)gj * p.ix + gi, nc, um, uh);
+    if (ions) {
+#pragma unroll
+      for (int n = 0; n < NVM; ++n) um[n] = src[n * sp];
+    }
+    if (neutrals) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) uh[n] = src[(NVM + n) * sp];
+    }
     if (COL) {
       // set_coefficients (Solver_rot.f90:62) rewrites the energies before set_flux: in
       // set_collisional and again in set_IR
@@ -718,11 +713,28 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       if (p.col_type) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
       if (p.irs) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
     }
-    to_prim<NVM>(um, uh, vm, vh, p);
+    if (ions) {
+      to_prim_mhd<NVM>(um, vm, p);
 #pragma unroll
-    for (int n = 0; n < NVM; ++n) sV[n * RR + idx] = vm[n];
+      for (int n = 0; n < NVM; ++n) sV[n * RR + idx] = vm[n];
+    }
+    if (neutrals) {
+      to_prim_hd(uh, vh, p);
 #pragma unroll
-    for (int n = 0; n < 5; ++n) sV[(NVM + n) * RR + idx] = vh[n];
+      for (int n = 0; n < 5; ++n) sV[(NVM + n) * RR + idx] = vh[n];
+    }
+  };
+  for (int u = tid; u < (SPLITP ? 2 : 1) * RR; u += NT) {
+    const int idx = SPLITP && u >= RR ? u - RR : u;
+    const bool ions = !SPLITP || u < RR, neutrals = !SPLITP || u >= RR;
+    const int ri = idx % RX, rj = idx / RX;
+    // the corners only for the curl of B next to the tile's corner faces (resistivity)
+    if (NDIM == 2 && !RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH))
+      continue;
+    const int gi = i0 - kH + ri, gj = NDIM == 2 ? j0 - kH + rj : 0;
+    if (gi >= p.ix || gj >= p.jx) continue;
+    if (NDIM == 2 && staged) convert(sV + idx, RR, idx, ions, neutrals);
+    else convert(Us + (long long)gj * p.ix + gi, nc, idx, ions, neutrals);
   }
   __syncthreads();
   // resi 2, stage 2: cfl_resi's bound over this tile's interior cells with the eta of this
@@ -751,9 +763,15 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     __syncthreads();
   }
 
-  // ---- 2. face fluxes (set_flux): x faces then y faces of the tile
   const int iend = p.m0 + p.nx, jend = NDIM == 2 ? p.m1 + p.ny : 1;
-  for (int f = tid; f < NFX + NFY; f += NT) {
+  const int ti = tid % TX, tj = tid / TX;
+  const int gi = i0 + ti, gj = j0 + tj;
+  const bool valid = tj < TY && gi < iend && (NDIM == 1 || gj < jend);
+
+  // ---- 2. face fluxes (set_flux): x faces then y faces of the tile
+  const bool ion_faces = S == 0 || tid < NI, neutral_faces = S == 0 || tid >= NI;
+  const int f0 = S == 1 && tid >= NI ? tid - NI : tid;
+  for (int f = f0; f < NFX + NFY; f += NI) {
     int a, s, perm_y;
     double *Fout;
     int fo, nf;
@@ -776,7 +794,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       fo = g;
       nf = NFY;
     }
-    {
+    if (ion_faces) {
       double vl[NVM], vr[NVM], fx[NVM];
 #pragma unroll
       for (int n = 0; n < NVM; ++n) {
@@ -794,7 +812,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         Fout[dst * nf + fo] = fx[n];
       }
     }
-    {
+    if (neutral_faces) {
       double vl[5], vr[5], fx[5];
 #pragma unroll
       for (int n = 0; n < 5; ++n) {
@@ -815,7 +833,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   if (RES) {
     // resistive_flux's terms, added by the thread that wrote the face's flux (same faces
     // per thread as above), in a loop of their own to keep the Riemann solvers' registers
-    for (int f = tid; f < NFX + NFY; f += NT) {
+    for (int f = S == 1 && tid >= NI ? NFX + NFY : tid; f < NFX + NFY; f += NI) {
       int a, s, nf, fo, e0, e1;
       double *Fout;
       const bool ydir = f >= NFX;
@@ -849,9 +867,6 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   __syncthreads();
 
   // ---- 3. per-cell source, update, epilogue
-  const int ti = tid % TX, tj = tid / TX;
-  const int gi = i0 + ti, gj = j0 + tj;
-  const bool valid = tj < TY && gi < iend && (NDIM == 1 || gj < jend);
   double dtc = 10.0, rhoc = 0.0, grc = 0.0;
   if (valid) {
     const long long q = (long long)gj * p.ix + gi;
@@ -1096,17 +1111,19 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     if (STAGE == 2 && COL && p.col_type) {
       // the alpha_c field that the next cfl reads (cfl_pn_col, Scheme_rot.f90:305-313)
       p.acf[q] = ac_s;
-      if (near_boundary<NDIM>(p, gi, gj)) write_ghosts<NDIM>(p, gi, gj, p.acf, 1, true);
+      if (near_boundary<NDIM>(p, gi, gj)) {
+        const double v[1] = {ac_s};
+        write_ghosts<NDIM, 1, false>(p, gi, gj, p.acf, v);
+      }
     }
   }
   if (STAGE == 2 && COL && p.col_type) exchanged_ghost_ac<NDIM, NVM, TX, TY, NT>(p, Us, i0, j0, tid, by, nby);
   if (STAGE == 2 && s_epi == 2) {
     if (RES && p.resi == 2) dtc = fmin(dtc, rb);  // the next step's cfl_resi
-    block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, (int)((s_step + 1) & 1));
+    block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, s_slot);
   }
-  if (STAGE == 2 && dt_mode == 1) {
-    // end of step, done by the last block to finish (every block has read the control
-    // block by then): time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636)
+  if (STAGE == 2 && RES && dt_mode == 1 && p.resi == 2) {
+    // end of step, by the last block to finish: the time increment needs every block's bound
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -1114,17 +1131,14 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       if (atomicAdd(&ctrl->blocks_done, 1u) == nb - 1) {
         __threadfence();
         ctrl->blocks_done = 0u;
-        if (RES && p.resi == 2) {
-          // the cfl after run_solver lowers the global dt that time advances by to
-          // cfl_resi's bound of this stage's eta (main.f90:47,58; Scheme_rot.f90:298)
-          const double tn = ctrl->time + fmin(dt, bitsd(atomicOr(p.resi_bound, 0ull)));
-          ctrl->time = tn;
-          ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
-                        (ctrl->nsteps > 0 && s_step + 1 >= ctrl->nsteps)) ? 1 : 0;
-        } else {
-          ctrl->time = ctrl->time_next;
-        }
-        ctrl->step = s_step + 1;
+        // the cfl after run_solver lowers the global dt that time advances by to
+        // cfl_resi's bound of this stage's eta (main.f90:47,58; Scheme_rot.f90:298)
+        const double tn = ctrl->time + fmin(dt, bitsd(atomicOr(p.resi_bound, 0ull)));
+        const long long st = ctrl->step + 1;
+        ctrl->time = tn;
+        ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
+                      (ctrl->nsteps > 0 && st >= ctrl->nsteps)) ? 1 : 0;
+        ctrl->step = st;
         if (ctrl->last) ctrl->done = 1;
         if (dt <= 1.0e-12) {
           ctrl->done = 1;
@@ -1254,7 +1268,8 @@ __global__ void flux_kernel(const KParams p, const double *__restrict__ U, doubl
     for (int c = 0; c < 4; ++c) {
       double um[NVM], uh[5], vm[NVM], vh[5];
       load_cell<NVM>(U, qa + (c - 1) * s, nc, um, uh);
-      to_prim<NVM>(um, uh, vm, vh, p);
+      to_prim_mhd<NVM>(um, vm, p);
+      to_prim_hd(uh, vh, p);
       for (int n = 0; n < NVM; ++n) V[c][n] = vm[n];
       for (int n = 0; n < 5; ++n) V[c][NVM + n] = vh[n];
     }
@@ -1405,9 +1420,9 @@ __global__ void nan_kernel(const double *__restrict__ U, long long n, int *flag)
 
 // ---------------------------------------------------------------- host launchers
 
-template <int NDIM, int NVM, int X>
+template <int NDIM, int NVM, int X, int S>
 constexpr size_t stage_smem_bytes() {
-  constexpr int TX = Tile<NDIM>::TX, TY = Tile<NDIM>::TY;
+  constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY;
   constexpr int RR = (TX + 2 * kH) * (NDIM == 2 ? TY + 2 * kH : 1);
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
   constexpr int EN = (TX + 2) * (NDIM == 2 ? TY + 2 : 1);
@@ -1416,9 +1431,16 @@ constexpr size_t stage_smem_bytes() {
 
 template <int NDIM, int NVM, int STAGE, int X>
 static cudaError_t set_stage_attr_x() {
-  return cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)stage_smem_bytes<NDIM, NVM, X>());
+  const cudaError_t e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 0>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)stage_smem_bytes<NDIM, NVM, X, 0>());
+#if !PIP_HEAT_ONLY
+  if (e == cudaSuccess)
+    return cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 1>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)stage_smem_bytes<NDIM, NVM, X, 1>());
+#endif
+  return e;
 }
 
 template <int NDIM, int NVM, int STAGE>
@@ -1447,71 +1469,111 @@ static cudaError_t prepare() {
   return set_stage_attr<2, 9, 2>();
 }
 
-template <int NDIM, int NVM, int STAGE>
-static cudaError_t launch_stage_t(const KParams &p, const double *Us, const double *U0, double *Uo,
-                                  DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
-                                  const CUtensorMap *tm, int rows) {
-  constexpr int TX = Tile<NDIM>::TX, TY = Tile<NDIM>::TY, NT = Tile<NDIM>::NT;
+// Whether a grid takes the small tiles (Tile<., 1>): while they all run at once.
+#ifndef PIP_SMALL_TILES
+#define PIP_SMALL_TILES 296
+#endif
+static bool small_tiles(const KParams &p) {
+#if PIP_HEAT_ONLY
+  return false;
+#else
+  if (p.ndim == 1) return (p.nx + Tile<1, 1>::TX - 1) / Tile<1, 1>::TX <= PIP_SMALL_TILES;
+  return (long long)((p.nx + Tile<2, 1>::TX - 1) / Tile<2, 1>::TX) *
+             ((p.ny + Tile<2, 1>::TY - 1) / Tile<2, 1>::TY) <= PIP_SMALL_TILES;
+#endif
+}
+
+template <int NDIM, int NVM, int STAGE, int X, int S>
+static cudaError_t launch_tiles(const KParams &p, const double *Us, const double *U0, double *Uo,
+                                DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
+                                const CUtensorMap *tm, int rows) {
+  constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = Tile<NDIM, S>::NT;
   const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
   if (NDIM == 1) rows = 0;
   const int gy = rows == 0 ? nby : rows == 1 ? (nby < 2 ? nby : 2) : nby - 2;
   if (gy <= 0) return cudaSuccess;   // no rows between the first and the last
-  dim3 grid((p.nx + TX - 1) / TX, gy);
   CUtensorMap none;
   std::memset(&none, 0, sizeof none);
-  const CUtensorMap &map = tm ? *tm : none;
-  const int use = tm ? 1 : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((p.nx + TX - 1) / TX, gy);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = stage_smem_bytes<NDIM, NVM, X, S>();
+  cfg.stream = s;
+  // a programmatic dependent of the previous kernel: its set-up overlaps that one's tail
+  // (not for the rows of a split stage, which events order across streams)
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = rows == 0 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, stage_kernel<NDIM, NVM, STAGE, X, S>, p, Us, U0, Uo, ctrl, dt_mode,
+                            epi, tm ? *tm : none, tm ? 1 : 0, rows);
+}
+
+template <int NDIM, int NVM, int STAGE, int S>
+static cudaError_t launch_stage_t(const KParams &p, const double *Us, const double *U0, double *Uo,
+                                  DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
+                                  const CUtensorMap *tm, int rows) {
   switch ((p.col_type || p.irl ? 1 : 0) | (p.resi ? 2 : 0)) {
     case 0:
-      stage_kernel<NDIM, NVM, STAGE, 0><<<grid, NT, stage_smem_bytes<NDIM, NVM, 0>(), s>>>(
-          p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
-      break;
+      return launch_tiles<NDIM, NVM, STAGE, 0, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
     case 1:
-      stage_kernel<NDIM, NVM, STAGE, 1><<<grid, NT, stage_smem_bytes<NDIM, NVM, 1>(), s>>>(
-          p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
-      break;
+      return launch_tiles<NDIM, NVM, STAGE, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 #if !PIP_HEAT_ONLY
     case 2:
-      stage_kernel<NDIM, NVM, STAGE, 2><<<grid, NT, stage_smem_bytes<NDIM, NVM, 2>(), s>>>(
-          p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
-      break;
+      return launch_tiles<NDIM, NVM, STAGE, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
     default:
-      stage_kernel<NDIM, NVM, STAGE, 3><<<grid, NT, stage_smem_bytes<NDIM, NVM, 3>(), s>>>(
-          p, Us, U0, Uo, ctrl, dt_mode, epi, map, use, rows);
-      break;
+      return launch_tiles<NDIM, NVM, STAGE, 3, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 #else
     default:
       return cudaErrorInvalidValue;
 #endif
   }
-  return cudaGetLastError();
 }
 
-static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
-                                double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
-                                const CUtensorMap *tm, int rows) {
+template <int S>
+static cudaError_t launch_stage_s(const KParams &p, int stage, const double *Us, const double *U0,
+                                  double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
+                                  const CUtensorMap *tm, int rows) {
 #if PIP_HEAT_ONLY
   if (p.ndim != 2) return cudaErrorInvalidValue;
 #else
   if (p.ndim == 1) {
-    return stage == 1 ? launch_stage_t<1, 8, 1>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0)
-                      : launch_stage_t<1, 8, 2>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0);
+    return stage == 1 ? launch_stage_t<1, 8, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0)
+                      : launch_stage_t<1, 8, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0);
   }
 #endif
   if (p.nvm == 9)
-    return stage == 1 ? launch_stage_t<2, 9, 1>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
-                      : launch_stage_t<2, 9, 2>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
-  return stage == 1 ? launch_stage_t<2, 8, 1>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
-                    : launch_stage_t<2, 8, 2>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
+    return stage == 1 ? launch_stage_t<2, 9, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
+                      : launch_stage_t<2, 9, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
+  return stage == 1 ? launch_stage_t<2, 8, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
+                    : launch_stage_t<2, 8, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 }
 
+// The small tiles take whole stages only: the rows of a split stage are rows of the large
+// ones, whose map (tile_map makes one for the tiles of whole stages) such a context lacks.
+static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
+                                double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
+                                const CUtensorMap *tm, int rows) {
+#if !PIP_HEAT_ONLY
+  if (small_tiles(p)) {
+    if (rows == 0)
+      return launch_stage_s<1>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, 0);
+    tm = nullptr;
+  }
+#endif
+  return launch_stage_s<0>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
+}
+
+template <int S>
+static bool tile_map_s(const KParams &p, const double *U, CUtensorMap *map) {
+  constexpr int TX = Tile<2, S>::TX, RX = TX + 2 * kH, RY = Tile<2, S>::TY + 2 * kH;
+  return tma_tile_ok(U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), p.m0 - kH, TX, RX, RY) &&
+         tma_encode(map, U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), RX, RY);
+}
 static bool tile_map(const KParams &p, const double *U, CUtensorMap *map) {
   if (p.ndim != 2) return false;
-  constexpr int TX = Tile<2>::TX, TY = Tile<2>::TY;
-  if (!tma_tile_ok(U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), p.m0 - kH, TX, TX + 2 * kH,
-                   TY + 2 * kH))
-    return false;
-  return tma_encode(map, U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), TX + 2 * kH, TY + 2 * kH);
+  return small_tiles(p) ? tile_map_s<1>(p, U, map) : tile_map_s<0>(p, U, map);
 }
 
 static int grid_for(long long n, int threads) {
