@@ -507,7 +507,9 @@ int push_ctrl(pip_ctx *c) {
 
 // One RK stage of the context's precision form (rows: every tile row, or the first and
 // last / the middle ones, see Launchers::stage).
-cudaError_t do_stage(pip_ctx *c, int stage, int dt_mode, int epi, int rows = 0) {
+// rates_ready: set_IR type 4's rates of this stage's state are in place already.
+cudaError_t do_stage(pip_ctx *c, int stage, int dt_mode, int epi, int rows = 0,
+                     bool rates_ready = false) {
   if (c->mixed) {
     if (stage == 1)
       return pip::mixed_stage(c->kp, 1, c->Ahi, c->Ahi, nullptr, c->Bf, nullptr, c->ctrl, dt_mode,
@@ -520,8 +522,10 @@ cudaError_t do_stage(pip_ctx *c, int stage, int dt_mode, int epi, int rows = 0) 
     // stage, then hydrogen_excitation_update on the updated state (Solver_rot.f90:218-220)
     const double *Us = stage == 1 ? c->A : c->B;
     double *Uo = stage == 1 ? c->B : c->A;
-    cudaError_t e = c->L->nlev_rates(c->kp, Us, c->kp.col_type ? 1 : 0, c->kp.ir_type == 0 ? 1 : 0,
-                                     nullptr, c->ctrl, c->stream);
+    cudaError_t e = cudaSuccess;
+    if (!rates_ready)
+      e = c->L->nlev_rates(c->kp, Us, c->kp.col_type ? 1 : 0, c->kp.ir_type == 0 ? 1 : 0, nullptr,
+                           c->ctrl, c->stream);
     if (e != cudaSuccess) return e;
     e = c->L->stage(c->kp, stage, Us, c->A, Uo, c->ctrl, dt_mode, epi, c->stream,
                     c->tma ? (stage == 1 ? &c->tm_a : &c->tm_b) : nullptr, rows);
@@ -541,6 +545,10 @@ cudaError_t do_cfl(pip_ctx *c, int slot) {
   if (c->mixed) return pip::mixed_cfl(c->kp, c->Ahi, c->Alo, c->ctrl, slot, c->stream);
   if (c->kp.irn) {
     // the time loop's set_IR before the cfl, the cfl, then its type-4 terms
+    if (c->L->nlev_fused_cfl(c->kp)) {
+      const cudaError_t f = c->L->nlev_rates_cfl(c->kp, c->A, c->ctrl, slot, c->stream);
+      return f != cudaSuccess ? f : c->L->cfl(c->kp, c->A, c->ctrl, slot, c->stream);
+    }
     cudaError_t e = c->L->nlev_rates(c->kp, c->A, 0, 0, nullptr, c->ctrl, c->stream);
     if (e != cudaSuccess) return e;
     if ((e = c->L->cfl(c->kp, c->A, c->ctrl, slot, c->stream)) != cudaSuccess) return e;
@@ -906,10 +914,16 @@ static int run_loop(pip_ctx *c, int64_t nsteps, double t_end, double *time_out,
     // bound, so the next cfl's rewrite cannot be fused into stage 2 either.  set_IR type 4:
     // the rates, excitation-update and cfl kernels of the 6-level model sit between the
     // stages and the cfl calls.
+    // The default build's type 4 evaluates the rates of a state once: the cfl that opens a step
+    // and the step's stage 1 see the same populations and, unless one of the cfl's floors acted
+    // (h.floored), the same state up to rounding; the cfl after run_solver leaves no other trace
+    // than its rewrite, except after the last step, whose rates stay readable.
+    const bool once = c->kp.irn && c->L->nlev_fused_cfl(c->kp);
+    bool ready = once && !h.floored;
     long long n = 0;
     int total_it = 0;
     while (!halted) {
-      CK(do_stage(c, 1, 1, 0));
+      CK(do_stage(c, 1, 1, 0, 0, ready));
       CK(do_stage(c, 2, 1, 0));
       if (c->hc) {
         int it = 0, hst = 0;
@@ -919,13 +933,16 @@ static int run_loop(pip_ctx *c, int64_t nsteps, double t_end, double *time_out,
       }
       if (sync_ctrl_to_host(c)) return PIP_ERR_CUDA;
       if (h.nan_flag || h.status || h.step != n + 1) break;
-      CK(do_cfl(c, (int)(n & 1)));          // the cfl after run_solver (main.f90:47)
+      // the cfl after run_solver (main.f90:47)
+      if (once && !h.done) CK(c->L->cfl(c->kp, c->A, c->ctrl, (int)(n & 1), c->stream));
+      else CK(do_cfl(c, (int)(n & 1)));
       if (h.done) break;
       CK(do_cfl(c, (int)((n + 1) & 1)));    // the next step's cfl (main.f90:36)
       ++n;
       if (c->kp.irn) {
         if (sync_ctrl_to_host(c)) return PIP_ERR_CUDA;
         if (h.status) break;
+        ready = once && !h.floored;
       }
     }
     c->hc_iters = total_it;

@@ -115,6 +115,7 @@ struct DevCtrl {
   // Set by block 0 of stage 1 for stage 2, which does not read what its own block 0 changes
   // (step, time, done): whether the step is skipped, and the reduction slot of the next dt.
   int skip, slot;
+  int floored;                    // default build: a cfl since stage 1 found a cell at a floor
   unsigned int blocks_done;       // last-block-done counter of the stage-2 kernel (resi 2)
 };
 
@@ -151,6 +152,11 @@ struct Launchers {
   cudaError_t (*nlev_update)(const KParams &p, const double *U, const DevCtrl *ctrl, int stage,
                              cudaStream_t s);
   cudaError_t (*nlev_cfl)(const KParams &p, double *U, DevCtrl *ctrl, int slot, cudaStream_t s);
+  // nlev_rates_cfl: nlev_rates (no collision rewrite, no ion_pot) with nlev_cfl's terms, where
+  // nlev_fused_cfl says so; it comes before the cfl kernel and replaces both
+  bool (*nlev_fused_cfl)(const KParams &p);
+  cudaError_t (*nlev_rates_cfl)(const KParams &p, const double *U, DevCtrl *ctrl, int slot,
+                                cudaStream_t s);
 };
 
 const Launchers &launchers_fast();

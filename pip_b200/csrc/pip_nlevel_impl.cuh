@@ -187,6 +187,112 @@ __device__ __forceinline__ bool nl_cell(const KParams &p, const NlevConst &k, do
 #endif
 }
 
+#if PIP_FAST
+// Weights and rows of the interpolation at z for the default build: the rows by 16-byte loads,
+// the row index as a 32-bit number (tables of up to 2^31 rows; nl_weights otherwise).
+struct NlRow {
+  double w0, w1, w2;
+  double2 a, b, c, d, e, f;      // rows xindex .. xindex+2: (yn, E0), (E1, E2) each
+};
+__device__ __forceinline__ NlRow nl_row(const KParams &p, double z) {
+  const int n = (int)p.nl_ntab;
+  const double t = (z - p.nl_xmin) * p.nl_xsc;
+  int xi = __double2int_rd(t);
+  const double r = t - (double)xi;
+  // within 1e-9 of a row boundary the reference's quotient decides, as in nl_weights
+  if (r < 1.0e-9 || r > 1.0 - 1.0e-9) xi = __double2int_rd((z - p.nl_xmin) / p.nl_xrange * (double)n);
+  xi = min(max(xi, 1), n - 2);
+  const double2 *q = reinterpret_cast<const double2 *>(p.nl_tab + 4ll * (xi - 1));
+  NlRow w;
+  w.a = __ldg(q);
+  w.b = __ldg(q + 1);
+  w.c = __ldg(q + 2);
+  w.d = __ldg(q + 3);
+  w.e = __ldg(q + 4);
+  w.f = __ldg(q + 5);
+  const double *rt = p.nl_rtab + 4ll * (xi - 1);
+  const double2 r01 = __ldg(reinterpret_cast<const double2 *>(rt));
+  const double d0 = z - w.a.x, d1 = z - w.c.x, d2 = z - w.e.x;
+  w.w0 = d1 * d2 * r01.x;
+  w.w1 = d0 * d2 * r01.y;
+  w.w2 = d0 * d1 * __ldg(rt + 2);
+  return w;
+}
+__device__ __forceinline__ double nl_E0(const NlRow &w) {
+  return fma(w.w0, w.a.y, fma(w.w1, w.c.y, w.w2 * w.e.y));
+}
+__device__ __forceinline__ double nl_E1(const NlRow &w) {
+  return fma(w.w0, w.b.x, fma(w.w1, w.d.x, w.w2 * w.f.x));
+}
+__device__ __forceinline__ double nl_E2(const NlRow &w) {
+  return fma(w.w0, w.b.y, fma(w.w1, w.d.y, w.w2 * w.f.y));
+}
+
+// nl_cell for the default build.  The Boltzmann factors of the level pairs are quotients of
+// five exponentials exp(E_a/kT) (15 and five more otherwise), T^(-3/2) a cubed inverse
+// square root, the reciprocals of y and z Newton's.  colrat(a+1,b+1) goes to put(a, b, value)
+// as it is formed.
+template <typename F>
+__device__ __forceinline__ bool nl_cell_fast(const KParams &p, const NlevConst &k, double te, double ne,
+                                             const double (&nx)[6], double &gi, double &gr, F put) {
+  bool bad = false;
+  const double s = sqrt(8.0 * kNlKb * te / kNlPi / kNlMe);
+  const double ikt = 1.0 / (kNlKb * te);
+  const double pre0 = ne * s * (2.0 * kNlPi * (kNlA0 * kNlA0));
+  double ex[5], iex[5];          // exp(E_a/kT) and its inverse
+#pragma unroll
+  for (int a = 0; a < 5; ++a) {
+    ex[a] = exp(k.eion[a] * ikt);
+    iex[a] = 1.0 / ex[a];
+  }
+  const double h = rsqrt_nr(te * (2.0 * kNlPi * kNlMehat * kNlKbhat / kNlHhat / kNlHhat * kNlE14));
+  const double saha = ne * (h * h * h);
+  double si = 0.0, sr = 0.0;
+#pragma unroll
+  for (int a = 0; a < 5; ++a) {
+    put(a, a, 0.0);
+    const double ri = (double)(a + 1);
+    const double pre = pre0 * (ri * ri);
+#pragma unroll
+    for (int b = a + 1; b < 5; ++b) {
+      const double y = k.enn[a][b] * ikt, z = k.rnn[a][b] + y;
+      const double iy = rcp_(y), iz = rcp_(z);
+      const NlRow wy = nl_row(p, y);
+      const double y1 = nl_E1(wy), y2 = nl_E2(wy);
+      const NlRow wz = nl_row(p, z);
+      const double z1 = nl_E1(wz), z2 = nl_E2(wz);
+      const double ann = k.ann[a][b];
+      const double c = pre * k.ixrat[a][b] * (y * y) *
+                       fma(ann, fma(iy + 0.5, y1, -(iz + 0.5) * z1),
+                           (k.bnn[a][b] - ann * k.lgt[a][b]) * fma(y2, iy, -z2 * iz));
+      const double up = k.gwq[a][b] * c, down = c * (ex[b] * iex[a]);
+      put(a, b, up);
+      put(b, a, down);
+      bad |= up < 0.0 || down < 0.0;
+    }
+    const double y = k.eion[a] * ikt, z = k.rn[a] + y;
+    const double iy = rcp_(y), iz = rcp_(z);
+    const NlRow wy = nl_row(p, y);
+    const double y1 = nl_E1(wy), zy = nl_E0(wy) - 2.0 * y1 + nl_E2(wy);
+    const NlRow wz = nl_row(p, z);
+    const double z1 = nl_E1(wz), zz = nl_E0(wz) - 2.0 * z1 + nl_E2(wz);
+    const double an0 = k.an0[a];
+    const double c = pre * (y * y) *
+                     fma(an0, fma(y1, iy, -z1 * iz), (k.bn0[a] - an0 * k.lgi[a]) * (zy - zz));
+    const double up = c * ex[a], down = up * k.gwh[a] * saha * ex[a];
+    put(a, 5, up);
+    put(5, a, down);
+    bad |= c < 0.0 || up < 0.0 || down < 0.0;
+    si = si + fmax(nx[a] * up, 0.0);
+    sr = sr + fmax(nx[5] * down, 0.0);
+  }
+  put(5, 5, 0.0);
+  gi = si;
+  gr = sr;
+  return bad;
+}
+#endif
+
 // IRgetionpot (PIP_rot.f90:1162-1235) of one cell.
 __device__ __forceinline__ double nl_ionpot(const KParams &p, const NlevConst &k,
                                             const double (&cr)[36], const double (&nx)[6]) {
@@ -217,49 +323,6 @@ __global__ void nlev_ref_kernel(const __grid_constant__ KParams p, double *out) 
   nl_cell(p, k, p.nl_T0, p.nl_n0, nx, cr, gi, gr);
   for (int m = 0; m < 36; ++m) out[m] = cr[m];
   out[36] = gr;
-}
-
-// set_IR type 4 over every cell of U (ghosts included): get_Te_HD/MHD's energy rewrite
-// (after set_collisional's when colrw), colrat from Te_p*T0/tfac and rho_i*n0/n0fac, the
-// normalised rates Gm_ion/rho_n/Gm_rec_ref*t_ir and Gm_rec/rho_i/Gm_rec_ref*t_ir.  U itself
-// is not written: the kernels that follow make the same rewrites of their copies.
-// ipmode 1: ion_pot (source_PIP's IRgetionpot) from the new colrat; 2: from crref (the
-// prologue's block).
-template <int NVM>
-__global__ void __launch_bounds__(128) nlev_rates_kernel(const __grid_constant__ KParams p,
-                                                         const double *__restrict__ U, int colrw,
-                                                         int ipmode, const double *crref,
-                                                         DevCtrl *ctrl) {
-  const NlevConst &k = *p.nl_k;
-  const long long nc = p.nc;
-  bool bad = false;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nc;
-       q += (long long)gridDim.x * blockDim.x) {
-    double um[NVM], uh[5];
-    load_cell<NVM>(U, q, nc, um, uh);
-    double te_m, te_h, rm, rh;
-    if (colrw) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
-    get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
-    double nx[6], cr[36], gi, gr;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) nx[m] = p.nl_nex[q + m * nc];
-    bad |= nl_cell(p, k, te_m * p.nl_T0 / p.nl_tfac, um[0] * p.nl_n0 / p.nl_n0fac, nx, cr, gi, gr);
-#pragma unroll
-    for (int a = 0; a < 6; ++a)
-#pragma unroll
-      for (int b = 0; b < 6; ++b) p.nl_cr[q + (long long)(a + 6 * b) * nc] = cr[a * 6 + b];
-    p.irg[q] = gi / uh[0] / p.nl_gref * p.nl_tir;
-    p.irg[nc + q] = gr / um[0] / p.nl_gref * p.nl_tir;
-    if (ipmode == 1) {
-      p.nl_ip[q] = nl_ionpot(p, k, cr, nx);
-    } else if (ipmode == 2) {
-      double c0[36];
-#pragma unroll
-      for (int m = 0; m < 36; ++m) c0[m] = crref[m];
-      p.nl_ip[q] = nl_ionpot(p, k, c0, nx);
-    }
-  }
-  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicCAS(&ctrl->status, 0, 9);  // PIP_ERR_RATE
 }
 
 // colrat(a+1,b+1) of cell q.
@@ -294,6 +357,137 @@ __device__ __forceinline__ double nl_conv(const KParams &p, const double *U, int
   double c = nl_deriv<1>(p, v, q, i, j) * U[q + (NVM + 1) * nc] / rh;
   if (NDIM == 2) c = c + nl_deriv<2>(p, v, q, i, j) * U[q + (NVM + 2) * nc] / rh;
   return c;
+}
+
+#if PIP_FAST
+// nl_conv of the five levels for the default build: one reciprocal per direction.
+template <int DIR>
+__device__ __forceinline__ void nl_conv_dir(const KParams &p, long long q, int i, int j, double v,
+                                            double (&c)[5]) {
+  const int order = p.nl_deriv, w = order == 4 ? 2 : 1;
+  const long long s = DIR == 1 ? 1 : p.ix, nc = p.nc;
+  const int k = DIR == 1 ? i : j, n = DIR == 1 ? p.ix : p.jx;
+  if (order == 0 || k < w || k >= n - w) return;
+  const double f = v * rcp_((order == 4 ? 12.0 : 2.0) * (DIR == 1 ? p.dx[i] : p.dy[j]));
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    const double *x = p.nl_nex + m * nc + q;
+    const double d = x[s] - x[-s];
+    c[m] = fma(f, order == 4 ? 8.0 * d - (x[2 * s] - x[-2 * s]) : d, c[m]);
+  }
+}
+template <int NDIM, int NVM>
+__device__ __forceinline__ void nl_conv5(const KParams &p, const double *U, long long q, int i, int j,
+                                         double (&c)[5]) {
+  const long long nc = p.nc;
+  const double ir = rcp_(U[q + NVM * nc]);
+#pragma unroll
+  for (int m = 0; m < 5; ++m) c[m] = 0.0;
+  nl_conv_dir<1>(p, q, i, j, U[q + (NVM + 1) * nc] * ir, c);
+  if (NDIM == 2) nl_conv_dir<2>(p, q, i, j, U[q + (NVM + 2) * nc] * ir, c);
+}
+#endif
+
+// set_IR type 4 over every cell of U (ghosts included): get_Te_HD/MHD's energy rewrite
+// (after set_collisional's when colrw), colrat from Te_p*T0/tfac and rho_i*n0/n0fac, the
+// normalised rates Gm_ion/rho_n/Gm_rec_ref*t_ir and Gm_rec/rho_i/Gm_rec_ref*t_ir.  U itself
+// is not written: the kernels that follow make the same rewrites of their copies.
+// ipmode 1: ion_pot (source_PIP's IRgetionpot) from the new colrat; 2: from crref (the
+// prologue's block).
+//
+// MODE 0: this, with nl_cell.  The default build takes nl_cell_fast where no ion_pot is wanted:
+// MODE 1 the rates alone, MODE 2 also nlev_cfl_kernel's terms (flag_IR_type 1 or 2) into slot
+// `slot`, from the rates in registers instead of 38 planes read back.  (The convection's m/rho is the
+// same before and after the cfl's rewrite, floors included.)  Bound by FP64 latency: 16
+// warps per SM at 128 registers; Orszag-Tang 512^2, us a launch: 102 -> 63 (MODE 1) and 102 + 44
+// of nlev_cfl_kernel -> 79 (MODE 2); nlev_update_kernel, with one reciprocal per direction in its
+// convection, 39 -> 25.
+template <int NDIM, int NVM, int MODE>
+__global__ void __launch_bounds__(128, MODE == 0 ? 1 : 4) nlev_rates_kernel(const __grid_constant__ KParams p,
+                                                         const double *__restrict__ U, int colrw,
+                                                         int ipmode, const double *crref,
+                                                         DevCtrl *ctrl, int slot) {
+  const NlevConst &k = *p.nl_k;
+  const long long nc = p.nc;
+  bool bad = false;
+  double gmax = 0.0, nxmax = 1.0e-5;
+  const double cg = p.nl_tir / p.nl_gref;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nc;
+       q += (long long)gridDim.x * blockDim.x) {
+    double um[NVM], uh[5];
+    load_cell<NVM>(U, q, nc, um, uh);
+    double te_m, te_h, rm, rh;
+    if (colrw) get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
+    get_te<NVM>(um, uh, p, te_m, te_h, rm, rh);
+    double nx[6], gi, gr;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) nx[m] = p.nl_nex[q + m * nc];
+#if PIP_FAST
+    if constexpr (MODE != 0) {
+      // the populations' tendencies from the rates as they are formed
+      double dn[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+      bad |= nl_cell_fast(p, k, te_m * p.nl_T0 / p.nl_tfac, um[0] * p.nl_n0 / p.nl_n0fac, nx, gi, gr,
+                          [&](int a, int b, double v) {
+                            p.nl_cr[q + (long long)(a + 6 * b) * nc] = v;
+                            if (MODE == 2) {
+                              if (b < 5) dn[b < 5 ? b : 0] = fma(nx[a], v, dn[b < 5 ? b : 0]);
+                              if (a < 5) dn[a < 5 ? a : 0] = fma(-nx[a], v, dn[a < 5 ? a : 0]);
+                            }
+                          });
+      const double ion = gi * rcp_(uh[0]) * cg, rec = gr * rcp_(um[0]) * cg;
+      p.irg[q] = ion;
+      p.irg[nc + q] = rec;
+      if (MODE == 2) {
+        gmax = fmax(gmax, fmax(ion, rec));
+        const int i = (int)(q % p.ix), j = (int)(q / p.ix);
+        double cv[5];
+        nl_conv5<NDIM, NVM>(p, U, q, i, j, cv);
+#pragma unroll
+        for (int ii = 0; ii < 5; ++ii) nxmax = fmax(nxmax, fma(dn[ii], cg, -cv[ii]));
+      }
+      continue;
+    }
+#endif
+    double cr[36];
+    bad |= nl_cell(p, k, te_m * p.nl_T0 / p.nl_tfac, um[0] * p.nl_n0 / p.nl_n0fac, nx, cr, gi, gr);
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+#pragma unroll
+      for (int b = 0; b < 6; ++b) p.nl_cr[q + (long long)(a + 6 * b) * nc] = cr[a * 6 + b];
+    p.irg[q] = gi / uh[0] / p.nl_gref * p.nl_tir;
+    p.irg[nc + q] = gr / um[0] / p.nl_gref * p.nl_tir;
+    if (ipmode == 1) {
+      p.nl_ip[q] = nl_ionpot(p, k, cr, nx);
+    } else if (ipmode == 2) {
+      double c0[36];
+#pragma unroll
+      for (int m = 0; m < 36; ++m) c0[m] = crref[m];
+      p.nl_ip[q] = nl_ionpot(p, k, c0, nx);
+    }
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicCAS(&ctrl->status, 0, 9);  // PIP_ERR_RATE
+  if (MODE == 2) {
+    // block maxima (exact), then one atomic per block on the ordered bits
+    __shared__ double red[2][4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      gmax = fmax(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+      nxmax = fmax(nxmax, __shfl_xor_sync(0xffffffffu, nxmax, o));
+    }
+    if (threadIdx.x % 32 == 0) {
+      red[0][threadIdx.x / 32] = gmax;
+      red[1][threadIdx.x / 32] = nxmax;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 4; ++w) {
+        gmax = fmax(gmax, red[0][w]);
+        nxmax = fmax(nxmax, red[1][w]);
+      }
+      atomicMax(&ctrl->red_gr[slot], dbits(gmax));
+      atomicMax(&ctrl->red_nx[slot], dbits(nxmax));
+    }
+  }
 }
 
 // hydrogen_excitation_update after a stage (Solver_rot.f90:218-220) over the interior cells
@@ -336,10 +530,16 @@ __global__ void __launch_bounds__(128) nlev_update_kernel(const __grid_constant_
 #pragma unroll
       for (int jj = 0; jj < 5; ++jj)
         d[ii] = d[ii] + PIP_NL_GT(nx[jj] * nl_cr(p, q, jj, ii)) - PIP_NL_GT(nx[ii] * nl_cr(p, q, ii, jj));
-    double o[6];
+    double o[6], cv[5];
+#if PIP_FAST
+    nl_conv5<NDIM, NVM>(p, U, q, i, j, cv);
+#else
+#pragma unroll
+    for (int ii = 0; ii < 5; ++ii) cv[ii] = nl_conv<NDIM, NVM>(p, U, ii, q, i, j);
+#endif
 #pragma unroll
     for (int ii = 0; ii < 5; ++ii) {
-      const double v = nx[ii] + dts * (d[ii] - nl_conv<NDIM, NVM>(p, U, ii, q, i, j));
+      const double v = nx[ii] + dts * (d[ii] - cv[ii]);
       o[ii] = v > kNlFloor ? v : kNlFloor;
     }
     const double tot = o[0] + o[1] + o[2] + o[3] + o[4] - U[q + NVM * nc];

@@ -645,6 +645,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   const double dt = s_dt, cmax = s_cmax;
   if (STAGE == 1 && block0 && tid == 0) {
     ctrl->skip = 0;
+    ctrl->floored = 0;
     if (dt_mode == 1) {
       // loop bookkeeping of main.f90:31,58 for this step (no block of stage 1 reads these)
       const long long st = ctrl->step;
@@ -1151,12 +1152,13 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 
 // cfl (Scheme_rot.f90:183-213) as a standalone pass over every cell: cq2pv rewrite of
 // both species in place, CFL candidates of interior cells, rho*alpha_c and IR maxima of all
-// cells into reduction slot `slot`.
+// cells into reduction slot `slot`.  The default build notes in ctrl->floored that a floor acted.
 template <int NVM>
-__global__ void __launch_bounds__(256) cfl_kernel(const KParams p, double *U, DevCtrl *ctrl,
-                                                  int slot) {
+__global__ void __launch_bounds__(256) cfl_kernel(const __grid_constant__ KParams p, double *U,
+                                                  DevCtrl *ctrl, int slot) {
   const double gm = p.gm;
   double dtc = 10.0, rhoc = 0.0, grc = 0.0;
+  bool floored = false;
   // cfl_resi with the eta of the last set_resistivity (resi 2; a fixed field's bound is
   // seeded into the slot by the host)
   if (p.resi == 2 && blockIdx.x == 0 && threadIdx.x == 0) dtc = bitsd(*p.resi_bound);
@@ -1165,27 +1167,49 @@ __global__ void __launch_bounds__(256) cfl_kernel(const KParams p, double *U, De
     double um[NVM], uh[5];
     load_cell<NVM>(U, q, nc, um, uh);
     double gp1 = 0.0, gp2 = 0.0;
-    if (p.irl) {                                        // the time loop's set_IR before cfl
+    const int i = (int)(q % p.ix), j = (int)(q / p.ix);
+    const bool interior = i >= p.m0 && i < p.ix - p.m0 && j >= p.m1 && j < p.jx - p.m1;
+    auto set_ir = [&]() {                               // the time loop's set_IR before cfl
       set_ir_cell<NVM>(um, uh, p, gp1, gp2);
       if (p.irf) {
         p.irg[q] = gp2;
         p.irg[nc + q] = gp1;
       }
+    };
+#if PIP_FAST
+    // away from the floors the rewrites are the identity up to rounding: nothing is written
+    double im, ih;
+    Prim<double> qm = prim_mhd<NVM>(um, gm, im), qh = prim_hd(uh, gm, ih);
+    const bool above = above_floors(qm, p.ro_lim, p.pr_lim) && above_floors(qh, p.ro_lim, p.pr_lim);
+    if (p.irl) set_ir();
+    if (!above) {
+      floored = true;
+      qm = rt_mhd<NVM>(um, p);
+      qh = rt_hd(uh, p);
+#pragma unroll
+      for (int n = 0; n < 5; ++n) U[q + n * nc] = um[n];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) U[q + (NVM + n) * nc] = uh[n];
     }
+    if (interior) {
+      const double gmin = fmin(fmin(p.dx[i], p.dy[j]), p.dz0);
+      dtc = fmin(dtc, cfl_cell_fast(qm, qh, um[5], um[6], um[7], gm, p.safety * gmin));
+    }
+#else
+    if (p.irl) set_ir();
     const Prim<double> qm = rt_mhd<NVM>(um, p);
     const Prim<double> qh = rt_hd(uh, p);
 #pragma unroll
     for (int n = 0; n < 5; ++n) U[q + n * nc] = um[n];
 #pragma unroll
     for (int n = 0; n < 5; ++n) U[q + (NVM + n) * nc] = uh[n];
-    const int i = (int)(q % p.ix), j = (int)(q / p.ix);
-    const bool interior = i >= p.m0 && i < p.ix - p.m0 && j >= p.m1 && j < p.jx - p.m1;
     if (interior) {
       const double gmin = fmin(fmin(p.dx[i], p.dy[j]), p.dz0);
       const double sg = p.safety * gmin;
       dtc = fmin(dtc, fmin(cfl_mhd_cell<double>(qm, um[5], um[6], um[7], gm, sg),
                            cfl_hd_cell<double>(qh, gm, sg)));
     }
+#endif
     if (!p.col_type) {
       rhoc = fmax(rhoc, fmax(um[0] * p.ac, uh[0] * p.ac));
     } else {
@@ -1200,6 +1224,7 @@ __global__ void __launch_bounds__(256) cfl_kernel(const KParams p, double *U, De
       grc = fmax(grc, fmax(g1, g2));
     }
   }
+  if (floored) ctrl->floored = 1;
   block_reduce_cfl<256>(dtc, rhoc, grc, ctrl, slot);
 }
 
@@ -1631,12 +1656,39 @@ static cudaError_t launch_nlev_ref(const KParams &p, double *out, cudaStream_t s
   return cudaGetLastError();
 }
 
+template <int MODE>
+static cudaError_t launch_rates_mode(const KParams &p, const double *U, int colrw, int ipmode,
+                                     const double *crref, DevCtrl *ctrl, int slot, cudaStream_t s) {
+  const int g = grid_for(p.nc, 128);
+  if (p.ndim == 1)
+    nlev_rates_kernel<1, 8, MODE><<<g, 128, 0, s>>>(p, U, colrw, ipmode, crref, ctrl, slot);
+  else if (p.nvm == 9)
+    nlev_rates_kernel<2, 9, MODE><<<g, 128, 0, s>>>(p, U, colrw, ipmode, crref, ctrl, slot);
+  else
+    nlev_rates_kernel<2, 8, MODE><<<g, 128, 0, s>>>(p, U, colrw, ipmode, crref, ctrl, slot);
+  return cudaGetLastError();
+}
+// nl_cell_fast indexes the table with 32 bits
+static bool fast_rates(const KParams &p) { return PIP_FAST && p.nl_ntab <= 0x7fffffffll; }
+
 static cudaError_t launch_nlev_rates(const KParams &p, const double *U, int colrw, int ipmode,
                                      const double *crref, DevCtrl *ctrl, cudaStream_t s) {
-  const int g = grid_for(p.nc, 128);
-  if (p.nvm == 9) nlev_rates_kernel<9><<<g, 128, 0, s>>>(p, U, colrw, ipmode, crref, ctrl);
-  else nlev_rates_kernel<8><<<g, 128, 0, s>>>(p, U, colrw, ipmode, crref, ctrl);
-  return cudaGetLastError();
+#if PIP_FAST
+  if (ipmode == 0 && fast_rates(p)) return launch_rates_mode<1>(p, U, colrw, 0, nullptr, ctrl, 0, s);
+#endif
+  return launch_rates_mode<0>(p, U, colrw, ipmode, crref, ctrl, 0, s);
+}
+
+// The time loop's set_IR before a cfl together with cfl_pip_ir_nexcite's terms; false where
+// the flavour or flag_IR_type 0 (whose ion_pot terms follow the cfl's rewrite) keeps them apart.
+static bool nlev_fused_cfl(const KParams &p) { return fast_rates(p) && p.ir_type != 0; }
+static cudaError_t launch_nlev_rates_cfl(const KParams &p, const double *U, DevCtrl *ctrl, int slot,
+                                         cudaStream_t s) {
+#if PIP_FAST
+  return launch_rates_mode<2>(p, U, 0, 0, nullptr, ctrl, slot, s);
+#else
+  return cudaErrorInvalidValue;
+#endif
 }
 
 static cudaError_t launch_nlev_update(const KParams &p, const double *U, const DevCtrl *ctrl,
@@ -1672,7 +1724,8 @@ const Launchers &PIP_LAUNCHERS() {
                               PIP_FLAVOUR::launch_nan,    PIP_FLAVOUR::launch_coefficients,
                               PIP_FLAVOUR::tile_map,      PIP_FLAVOUR::launch_nlev_ref,
                               PIP_FLAVOUR::launch_nlev_rates, PIP_FLAVOUR::launch_nlev_update,
-                              PIP_FLAVOUR::launch_nlev_cfl};
+                              PIP_FLAVOUR::launch_nlev_cfl, PIP_FLAVOUR::nlev_fused_cfl,
+                              PIP_FLAVOUR::launch_nlev_rates_cfl};
   return L;
 }
 
