@@ -110,12 +110,11 @@ struct RowFactors {
 
 // The nine entries of row (i,j), in the reference's neighbour order 0 (i,j), 1 (i-1,j),
 // 2 (i+1,j), 3 (i,j-1), 4 (i,j+1), 5 (i-1,j-1), 6 (i+1,j-1), 7 (i-1,j+1), 8 (i+1,j+1),
-// with set_matrix_boundary's folds (HC_rot.f90:468-529) on the sides without a neighbouring
-// rank (boundary type 0 marks an exchanged face: pip_set_neighbors).  One rank per
-// direction: every side folds (MPI_rot.f90:123).
+// before set_matrix_boundary's folds (HC_rot.f90:468-529), which folds() makes on the sides
+// without a neighbouring rank (boundary type 0 marks an exchanged face: pip_set_neighbors).
+// One rank per direction: every side folds (MPI_rot.f90:123).
 template <typename T>
-__device__ __forceinline__ void entries(const KParams &p, const RowFactors<T> &f, int i, int j,
-                                        T (&c)[9]) {
+__device__ __forceinline__ void entries(const RowFactors<T> &f, T (&c)[9]) {
   const T eta = f.eta;
   const T exy = eta * (T(0.25) * f.idx * f.idy);
   const T bxxl = -(eta * f.fxxl * f.cxl);
@@ -135,6 +134,11 @@ __device__ __forceinline__ void entries(const KParams &p, const RowFactors<T> &f
   c[7] = -(bxyl + byxu);
   c[8] = bxyr + byxu;
   c[0] = T(1) - (c[1] + c[2] + c[3] + c[4]);
+}
+
+// The folds of row (i,j).
+template <typename T>
+__device__ __forceinline__ void folds(const KParams &p, int i, int j, T (&c)[9]) {
   if (i == p.m0 && p.typex[0] != 0) {                 // x-minus
     c[0] = c[1] + c[0]; c[1] = T(0);
     c[3] = c[3] + c[5]; c[5] = T(0);
@@ -157,19 +161,19 @@ __device__ __forceinline__ void entries(const KParams &p, const RowFactors<T> &f
   }
 }
 
-// w is the 3x3 neighbourhood [dj+1][di+1] of a vector; sum_n c_n * w_n, n = 0..8 left to
-// right, in T.
+// d, m, u are the rows j-1, j, j+1 of a vector at columns i-1, i, i+1; sum_n c_n * w_n,
+// n = 0..8 left to right, in T.
 template <typename T>
-__device__ __forceinline__ T stencil(const T (&c)[9], const T (&w)[3][3]) {
-  T s = c[0] * w[1][1];
-  s = s + c[1] * w[1][0];
-  s = s + c[2] * w[1][2];
-  s = s + c[3] * w[0][1];
-  s = s + c[4] * w[2][1];
-  s = s + c[5] * w[0][0];
-  s = s + c[6] * w[0][2];
-  s = s + c[7] * w[2][0];
-  s = s + c[8] * w[2][2];
+__device__ __forceinline__ T stencil(const T (&c)[9], const T (&d)[3], const T (&m)[3], const T (&u)[3]) {
+  T s = c[0] * m[1];
+  s = s + c[1] * m[0];
+  s = s + c[2] * m[2];
+  s = s + c[3] * d[1];
+  s = s + c[4] * u[1];
+  s = s + c[5] * d[0];
+  s = s + c[6] * d[2];
+  s = s + c[7] * u[0];
+  s = s + c[8] * u[2];
   return s;
 }
 
@@ -377,8 +381,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 //                                                        formed from these at each point
 //   own vectors    (row j, columns i0 .. i0+SX-1)
 //   eta (row j), fxx and fxy (row j, columns i0 .. i0+SX: both x-faces of every cell),
-//   fyy and fyx (rows j and j+1: both y-faces).
-// Window rows ja-1 and ja come from plain loads before the pipeline starts.  A segment is
+//   fyy and fyx (row j+1: the upper y-face; the lower one is kept from the row before).
+// Window rows ja-1 and ja and the lower faces of row ja come from plain loads before the
+// pipeline starts.  A segment is
 // copied from its start rounded down to 16 bytes, its length rounded up to 16 bytes and cut
 // at the end of its allocation (conduction runs with at least two ghost rows, so the cut
 // never reaches a value that is used).
@@ -388,7 +393,7 @@ template <> struct KindShape<KINIT> { static constexpr int nw = 1, no = 1; };  /
 template <> struct KindShape<K1> { static constexpr int nw = 3, no = 2; };     // p, Ap, r | r, r0
 template <> struct KindShape<K2> { static constexpr int nw = 2, no = 0; };     // r, Ap' |
 template <> struct KindShape<K3> { static constexpr int nw = 3, no = 2; };     // x, p', t | b, r0
-constexpr int kMatCopies = 7;
+constexpr int kMatCopies = 5;
 
 template <int KIND>
 __host__ __device__ constexpr int n_copies() {
@@ -425,10 +430,9 @@ __device__ __forceinline__ void copy_desc(const BicgArgs<T> &a, long long nc, in
   } else if (c < NW + NO) {
     base = a.o[c - NW]; dj = 0; di = 0; n = SX; lim = a.o[c - NW] + nc;
   } else {
-    const int k = c - NW - NO;     // eta, fxx, fxy, fyy(j), fyy(j+1), fyx(j), fyx(j+1)
-    const int plane = k == 0 ? 0 : (k <= 2 ? k : (k <= 4 ? 3 : 4));
-    base = a.m + plane * nc;
-    dj = (k == 4 || k == 6) ? 1 : 0;
+    const int k = c - NW - NO;     // eta, fxx, fxy, fyy(j+1), fyx(j+1)
+    base = a.m + k * nc;
+    dj = k >= 3 ? 1 : 0;
     di = 0;
     n = (k == 1 || k == 2) ? SX + 1 : SX;
     lim = a.m + NPL * nc;
@@ -445,9 +449,20 @@ __device__ __forceinline__ void copy_desc(const BicgArgs<T> &a, long long nc, in
 // the copies it issued land before the block leaves.
 constexpr int kConsumerWarps = SX / 32;
 constexpr int kBlock = SX + 32;
+template <typename T>
+__host__ __device__ constexpr int blocks_per_sm() {
+  return sizeof(T) == 4 ? 7 : 4;
+}
 
-template <typename T, int KIND>
-__global__ void __launch_bounds__(kBlock) bicg_kernel(const __grid_constant__ KParams p,
+// Consumer warps: the vector's rows j-1, j, j+1 rotate through three register rows (the row loop
+// is unrolled by three groups, so no row is copied), the grid factors of the next row are
+// loaded a row ahead, and the folds are one branch that only edge cells take.  Where every
+// plane starts on a 16-byte boundary (UNI: nc times the element size is a multiple of 16, all
+// but grids of odd ix and jx), the copies of a row start at one of three offsets in their
+// segments, kept in registers; else the producer hands the offsets over.  Instructions, not
+// HBM, bound these kernels (issue 53 %, DRAM 48-58 % before).  KH 2048x1024, FP64: HC_US.
+template <typename T, int KIND, bool UNI>
+__global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const __grid_constant__ KParams p,
                                                      const __grid_constant__ BicgArgs<T> a) {
   constexpr int NW = KindShape<KIND>::nw, NO = KindShape<KIND>::no;
   constexpr int NCP = n_copies<KIND>();
@@ -458,7 +473,7 @@ __global__ void __launch_bounds__(kBlock) bicg_kernel(const __grid_constant__ KP
       reinterpret_cast<unsigned long long *>(smem + (size_t)NS * RS * NCP * SLOT * sizeof(T));
   unsigned long long *empty = full + NS;
   static_assert(RS * NCP <= 32, "one lane of the producer warp per staged copy");
-  __shared__ int off[NS][RS][NCP];
+  __shared__ int off[UNI ? 1 : NS][RS][NCP];
   __shared__ volatile int s_fault;
 
   const int t = threadIdx.x;
@@ -533,7 +548,7 @@ __global__ void __launch_bounds__(kBlock) bicg_kernel(const __grid_constant__ KP
         uintptr_t end = (ad + c_len + 15) & ~(uintptr_t)15;
         if (end > c_cap) end = c_cap;
         bytes = (uint32_t)(end - a0);
-        off[st][lrow][lcopy] = (int)((ad - a0) / sizeof(T));
+        if (!UNI) off[st][lrow][lcopy] = (int)((ad - a0) / sizeof(T));
       }
       uint32_t total = bytes;
 #pragma unroll
@@ -574,8 +589,11 @@ __global__ void __launch_bounds__(kBlock) bicg_kernel(const __grid_constant__ KP
       return v[0] + s1 * v[1] + s2 * v[2];
     };
 
-    T w[3][3];
+    T w[3][3];                    // row r: w[r % 3] is row j-1, the next ones j and j+1
     RowFactors<T> f;
+    const T *gy = a.g + 3 * ix;
+    T cyd = T(0), cyu = T(0), idy = T(0);      // grid factors of the row to come
+    f.fyyu = f.fyxu = T(0);
     if (active && nrows > 0) {
 #pragma unroll
       for (int dr = 0; dr < 2; ++dr)
@@ -590,100 +608,129 @@ __global__ void __launch_bounds__(kBlock) bicg_kernel(const __grid_constant__ KP
       f.cxl = a.g[i];
       f.cxr = a.g[ix + i];
       f.idx = a.g[2 * ix + i];
+      const T *mr = a.m + (long long)ja * ix + i;
+      f.fyyu = mr[3 * nc];
+      f.fyxu = mr[4 * nc];
+      cyd = gy[ja];
+      cyu = gy[p.jx + ja];
+      idy = gy[2 * p.jx + ja];
     }
-    const T *gy = a.g + 3 * ix;
+    const bool edge_x = (i == p.m0 && p.typex[0] != 0) || (i == p.m0 + p.nx - 1 && p.typex[1] != 0);
+    const int j_lo = p.typey[0] != 0 ? p.m1 : -1, j_hi = p.typey[1] != 0 ? p.m1 + p.ny - 1 : -1;
+    constexpr int AL = 16 / (int)sizeof(T) - 1;             // elements past a 16-byte boundary
+    int at = (int)(((long long)ja * ix + i0) & AL);         // UNI: of (row, i0)
+    const int step = (int)(ix & AL);
+    long long q = (long long)ja * ix + i;
     const int lane = t & 31;
-    for (int g = 0; g < ngroups; ++g) {
-      const int st = g % NS;
-      bool ok = false;
-      for (int k = 0; k < wait_limit && !ok; ++k) {
-        ok = mbar_try_wait(smem_addr(&full[st]), (uint32_t)((g / NS) & 1));
-        if (!ok && s_fault) break;
-      }
-      if (!__all_sync(0xffffffffu, ok)) {
-        if (lane == 0) s_fault = 1;
-        break;
-      }
+    int st = 0, phase = 0;
+    bool stop = false;
+    for (int g0 = 0; g0 < ngroups && !stop; g0 += 3) {
 #pragma unroll
-      for (int rr = 0; rr < RS; ++rr) {
-        const int r = g * RS + rr, j = ja + r;
-        if (r >= nrows) break;
-        const T *sb = buf + (size_t)(st * RS + rr) * NCP * SLOT;
-        const int *of = off[st][rr];
-        if (active) {
-          const long long q = (long long)j * ix + i;
+      for (int k = 0; k < 3; ++k) {
+        const int g = g0 + k;
+        if (g >= ngroups) break;
+        bool ok = false;
+        for (int n = 0; n < wait_limit && !ok; ++n) {
+          ok = mbar_try_wait(smem_addr(&full[st]), (uint32_t)phase);
+          if (!ok && s_fault) break;
+        }
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) s_fault = 1;
+          stop = true;
+          break;
+        }
 #pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            T v[3];
+        for (int rr = 0; rr < RS; ++rr) {
+          const int r = g * RS + rr, j = ja + r;
+          if (r >= nrows) break;
+          const int z = (k * RS + rr) % 3;
+          T (&wd)[3] = w[z], (&wm)[3] = w[(z + 1) % 3], (&wu)[3] = w[(z + 2) % 3];
+          const T *sb = buf + (size_t)(st * RS + rr) * NCP * SLOT + t;
+          const int up = (at + step) & AL;
+          auto seg = [&](int c, int kind) -> const T * {    // copy c; kind 0 window, 1 own, 2 row j+1
+            if (UNI) return sb + c * SLOT + (kind == 0 ? ((up - 1) & AL) : kind == 1 ? at : up);
+            return sb + c * SLOT + off[st][rr][c];
+          };
+          if (active) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c] = c < NW ? sb[c * SLOT + of[c] + t + d] : T(0);
-            w[2][d] = form(v);
+            for (int d = 0; d < 3; ++d) {
+              T v[3];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) v[c] = c < NW ? seg(c, 0)[d] : T(0);
+              wu[d] = form(v);
+            }
+            T own[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) own[c] = c < NO ? seg(NW + c, 1)[0] : T(0);
+            constexpr int mc = NW + NO;
+            f.eta = seg(mc, 1)[0];
+            f.fxxl = seg(mc + 1, 1)[0];
+            f.fxxr = seg(mc + 1, 1)[1];
+            f.fxyl = seg(mc + 2, 1)[0];
+            f.fxyr = seg(mc + 2, 1)[1];
+            f.fyyd = f.fyyu;
+            f.fyyu = seg(mc + 3, 2)[0];
+            f.fyxd = f.fyxu;
+            f.fyxu = seg(mc + 4, 2)[0];
+            f.cyd = cyd;
+            f.cyu = cyu;
+            f.idy = idy;
+            if (r + 1 < nrows) {
+              cyd = gy[j + 1];
+              cyu = gy[p.jx + j + 1];
+              idy = gy[2 * p.jx + j + 1];
+            }
+            T c[9];
+            entries(f, c);
+            if (edge_x || j == j_lo || j == j_hi) folds(p, i, j, c);
+            if (KIND == KINIT) {
+              // r = b - A x term by term, as the reference's initial residual
+              const T bq = own[0];
+              T v = bq;
+              v = v - c[0] * wm[1];
+              v = v - c[1] * wm[0];
+              v = v - c[2] * wm[2];
+              v = v - c[3] * wd[1];
+              v = v - c[4] * wu[1];
+              v = v - c[5] * wd[0];
+              v = v - c[6] * wd[2];
+              v = v - c[7] * wu[0];
+              v = v - c[8] * wu[2];
+              a.out[0][q] = v;
+              a.out[1][q] = v;
+              a.out[2][q] = v;
+              acc0 += (double)v * (double)v;
+              acc1 += (double)bq * (double)bq;
+            } else if (KIND == K1) {
+              a.out[0][q] = wm[1];
+              const T av = stencil(c, wd, wm, wu);
+              a.out[1][q] = av;
+              const double r0q = (double)own[1];
+              acc0 += (double)own[0] * r0q;
+              acc1 += r0q * (double)av;
+            } else if (KIND == K2) {
+              a.out[0][q] = wm[1];
+              const T tv = stencil(c, wd, wm, wu);
+              acc0 += (double)wm[1] * (double)tv;
+              acc1 += (double)tv * (double)tv;
+            } else {
+              a.out[0][q] = wm[1];
+              const T v = own[0] - stencil(c, wd, wm, wu);
+              a.out[1][q] = v;
+              acc0 += (double)own[1] * (double)v;
+              acc1 += (double)v * (double)v;
+            }
           }
-          T own[2];
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-            own[c] = c < NO ? sb[(NW + c) * SLOT + of[NW + c] + t] : T(0);
-          constexpr int mc = NW + NO;
-          f.eta = sb[mc * SLOT + of[mc] + t];
-          f.fxxl = sb[(mc + 1) * SLOT + of[mc + 1] + t];
-          f.fxxr = sb[(mc + 1) * SLOT + of[mc + 1] + t + 1];
-          f.fxyl = sb[(mc + 2) * SLOT + of[mc + 2] + t];
-          f.fxyr = sb[(mc + 2) * SLOT + of[mc + 2] + t + 1];
-          f.fyyd = sb[(mc + 3) * SLOT + of[mc + 3] + t];
-          f.fyyu = sb[(mc + 4) * SLOT + of[mc + 4] + t];
-          f.fyxd = sb[(mc + 5) * SLOT + of[mc + 5] + t];
-          f.fyxu = sb[(mc + 6) * SLOT + of[mc + 6] + t];
-          f.cyd = gy[j];
-          f.cyu = gy[p.jx + j];
-          f.idy = gy[2 * p.jx + j];
-          T c[9];
-          entries(p, f, i, j, c);
-          if (KIND == KINIT) {
-            // r = b - A x term by term, as the reference's initial residual
-            const T bq = own[0];
-            T v = bq;
-            v = v - c[0] * w[1][1];
-            v = v - c[1] * w[1][0];
-            v = v - c[2] * w[1][2];
-            v = v - c[3] * w[0][1];
-            v = v - c[4] * w[2][1];
-            v = v - c[5] * w[0][0];
-            v = v - c[6] * w[0][2];
-            v = v - c[7] * w[2][0];
-            v = v - c[8] * w[2][2];
-            a.out[0][q] = v;
-            a.out[1][q] = v;
-            a.out[2][q] = v;
-            acc0 += (double)v * (double)v;
-            acc1 += (double)bq * (double)bq;
-          } else if (KIND == K1) {
-            a.out[0][q] = w[1][1];
-            const T av = stencil(c, w);
-            a.out[1][q] = av;
-            const double r0q = (double)own[1];
-            acc0 += (double)own[0] * r0q;
-            acc1 += r0q * (double)av;
-          } else if (KIND == K2) {
-            a.out[0][q] = w[1][1];
-            const T at = stencil(c, w);
-            acc0 += (double)w[1][1] * (double)at;
-            acc1 += (double)at * (double)at;
-          } else {
-            a.out[0][q] = w[1][1];
-            const T v = own[0] - stencil(c, w);
-            a.out[1][q] = v;
-            acc0 += (double)own[1] * (double)v;
-            acc1 += (double)v * (double)v;
-          }
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            w[0][d] = w[1][d];
-            w[1][d] = w[2][d];
-          }
+          at = up;
+          q += ix;
+        }
+        __syncwarp();                // the warp's reads of stage st are done
+        if (lane == 0) mbar_arrive(smem_addr(&empty[st]));
+        if (++st == NS) {
+          st = 0;
+          phase ^= 1;
         }
       }
-      __syncwarp();                // the warp's reads of stage st are done
-      if (lane == 0) mbar_arrive(smem_addr(&empty[st]));
     }
   }
   // the next kernel of the solve may start its launch (it waits for this one to complete
@@ -770,29 +817,29 @@ struct Grid {
 };
 
 template <typename T, int KIND>
-cudaError_t kind_blocks(int *bps) {
-  const size_t smem = stage_smem<T, KIND>();
-  cudaError_t err = cudaFuncSetAttribute(bicg_kernel<T, KIND>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int n = 0;
+cudaError_t set_smem() {
+  cudaError_t err = cudaFuncSetAttribute(bicg_kernel<T, KIND, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)stage_smem<T, KIND>());
   if (err == cudaSuccess)
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bicg_kernel<T, KIND>, kBlock, smem);
-  if (err == cudaSuccess) *bps = std::min(*bps, std::max(n, 1));
+    err = cudaFuncSetAttribute(bicg_kernel<T, KIND, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)stage_smem<T, KIND>());
   return err;
 }
 
 // The grid of the four kernels of precision T: as many row ranges per column block as fill
-// every SM at the occupancy of the most demanding kernel.
+// every SM with blocks_per_sm blocks.  The partition fixes the order of the dot products'
+// additions, and with it every iterate.
 template <typename T>
 cudaError_t make_grid(const KParams &k, int sms, Grid *g) {
-  int bps = 1 << 20;
-  cudaError_t err = kind_blocks<T, KINIT>(&bps);
-  if (err == cudaSuccess) err = kind_blocks<T, K1>(&bps);
-  if (err == cudaSuccess) err = kind_blocks<T, K2>(&bps);
-  if (err == cudaSuccess) err = kind_blocks<T, K3>(&bps);
+  cudaError_t err = set_smem<T, KINIT>();
+  if (err == cudaSuccess) err = set_smem<T, K1>();
+  if (err == cudaSuccess) err = set_smem<T, K2>();
+  if (err == cudaSuccess) err = set_smem<T, K3>();
   if (err != cudaSuccess) return err;
   g->ncb = (k.nx + SX - 1) / SX;
-  g->nrb = std::max(1, std::min(k.ny, sms * bps / g->ncb));
+  g->nrb = std::max(1, std::min(k.ny, sms * blocks_per_sm<T>() / g->ncb));
   g->nb = g->ncb * g->nrb;
   return cudaSuccess;
 }
@@ -812,7 +859,9 @@ void launch(const Grid &g, const KParams &k, BicgArgs<T> a, cudaStream_t s) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, bicg_kernel<T, KIND>, k, a);
+  // every plane is an allocation of its own or a multiple of nc elements into one
+  if (k.nc * (long long)sizeof(T) % 16 == 0) cudaLaunchKernelEx(&cfg, bicg_kernel<T, KIND, true>, k, a);
+  else cudaLaunchKernelEx(&cfg, bicg_kernel<T, KIND, false>, k, a);
 }
 
 template <typename T>
@@ -1207,7 +1256,8 @@ __global__ void __launch_bounds__(NT) spmv_kernel(const KParams p, const double 
     const long long q = (long long)j * p.ix + i;
     double w[3][3], c[9];
     window(p, v, q, w);
-    entries(p, factors(p, m, g, i, j), i, j, c);
+    entries(factors(p, m, g, i, j), c);
+    folds(p, i, j, c);
     if (KIND == 0) {
       const double bq = b[q];
       double x = bq;
@@ -1226,16 +1276,16 @@ __global__ void __launch_bounds__(NT) spmv_kernel(const KParams p, const double 
       a0 = x * x;
       a1 = bq * bq;
     } else if (KIND == 1) {
-      const double av = stencil(c, w);
+      const double av = stencil(c, w[0], w[1], w[2]);
       out[q] = av;
       a0 = r[q] * r0[q];
       a1 = r0[q] * av;
     } else if (KIND == 2) {
-      const double at = stencil(c, w);
+      const double at = stencil(c, w[0], w[1], w[2]);
       a0 = w[1][1] * at;
       a1 = at * at;
     } else {
-      const double x = b[q] - stencil(c, w);
+      const double x = b[q] - stencil(c, w[0], w[1], w[2]);
       r[q] = x;
       a0 = r0[q] * x;
       a1 = x * x;
