@@ -238,6 +238,58 @@ __device__ bool reduce2(double a, double b, double *part, unsigned int *counter,
   return true;
 }
 
+// Block sums of 2 values into part[k*nb + block], for sum_parts of the next kernel.
+template <int NTB>
+__device__ __forceinline__ void block_parts(double a, double b, double *part) {
+  __shared__ double s[2][NTB / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  const int w = threadIdx.x / 32;
+  if (threadIdx.x % 32 == 0) {
+    s[0][w] = a;
+    s[1][w] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double x = 0.0, y = 0.0;
+    for (int k = 0; k < NTB / 32; ++k) {
+      x += s[0][k];
+      y += s[1][k];
+    }
+    part[blockIdx.x] = x;
+    part[gridDim.x + blockIdx.x] = y;
+  }
+}
+
+// The totals of the previous kernel's block sums, by the first NR threads of every block, with
+// the additions in reduce2's order.
+template <int NR>
+__device__ __forceinline__ void sum_parts(const double *part, double (&tot)[2]) {
+  __shared__ double s2[2][NR];
+  const unsigned int nb = gridDim.x;
+  const int t = threadIdx.x;
+  double x = 0.0, y = 0.0;
+  for (unsigned int k = t; k < nb; k += NR) {
+    x += part[k];
+    y += part[nb + k];
+  }
+  s2[0][t] = x;
+  s2[1][t] = y;
+  asm volatile("bar.sync 1, %0;" ::"n"(NR) : "memory");
+  for (int h = NR / 2; h > 0; h >>= 1) {
+    if (t < h) {
+      s2[0][t] += s2[0][t + h];
+      s2[1][t] += s2[1][t + h];
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(NR) : "memory");
+  }
+  tot[0] = s2[0][0];
+  tot[1] = s2[1][0];
+}
+
 // cq2pv_mhd on every cell (rewrites the ion planes in place), te = gm*(pr/ro), and the
 // kinetic and magnetic energy terms of pv2cq_mhd for the conversion back.
 __global__ void setup_kernel(const KParams p, double *U, double *te, double *b, double *kin,
@@ -346,6 +398,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// Adds bytes to the current phase without an arrival.
+__device__ __forceinline__ void mbar_more_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -412,7 +469,8 @@ struct BicgArgs {
   const T *w[3];             // window vectors
   const T *o[2];             // own vectors
   T *out[3];                 // INIT: r, r0, p;  K1: p', Ap';  K2: t;  K3: x', r
-  double *part;
+  const double *part;        // K2, K3: the previous kernel's block sums
+  double *part_out;          // this kernel's
   Scal *sc;
   int ncb, nrb;              // column blocks, row ranges per column block
   cudaGraphConditionalHandle loop;  // k3 in the device-side loop: its while condition
@@ -496,9 +554,56 @@ __global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  // Launched as a programmatic dependent of the solve's previous kernel: everything above
-  // reads only the arguments; the vectors and scalars that kernel wrote are read after it
-  // has completed.
+  __syncthreads();
+  // producer: lane rr*NCP + c owns copy c of row rr of a group: its source address at row
+  // ja + rr, the length and the allocation end; the first element of that copy inside its
+  // staged segment goes to off[stage][rr][c] for the consumers (not UNI)
+  const int plane_lane = t - SX;
+  const int lrow = plane_lane / NCP, lcopy = plane_lane % NCP;
+  uintptr_t c_addr = 0, c_cap = 0;
+  uint32_t c_len = 0;
+  const bool owns = producer && plane_lane < RS * NCP, matrix = owns && lcopy >= NW + NO;
+  if (owns) {
+    const T *base, *lim;
+    int dj, di, n;
+    copy_desc<T, KIND>(a, nc, lcopy, base, dj, di, n, lim);
+    c_addr = (uintptr_t)(base + ((long long)(ja + lrow + dj) * ix + i0 + di));
+    c_len = (uint32_t)(n * sizeof(T));
+    c_cap = (uintptr_t)lim & ~(uintptr_t)15;
+  }
+  const uintptr_t row_bytes = (uintptr_t)ix * sizeof(T);
+  // the lane's copy of group g: source and length (0: none)
+  auto source = [&](int g, uintptr_t &a0) -> uint32_t {
+    if (!owns || g * RS + lrow >= nrows) return 0u;
+    const uintptr_t ad = c_addr + (uintptr_t)(g * RS) * row_bytes;
+    a0 = ad & ~(uintptr_t)15;
+    uintptr_t end = (ad + c_len + 15) & ~(uintptr_t)15;
+    if (end > c_cap) end = c_cap;
+    if (!UNI) off[g % NS][lrow][lcopy] = (int)((ad - a0) / sizeof(T));
+    return (uint32_t)(end - a0);
+  };
+  auto issue = [&](int g, bool mine, uintptr_t a0, uint32_t bytes) {
+    const int st = g % NS;
+    if (mine && bytes)
+      bulk_load(smem_addr(buf + ((size_t)(st * RS + lrow) * NCP + lcopy) * SLOT), (const void *)a0,
+                bytes, smem_addr(&full[st]));
+  };
+  // Launched as a programmatic dependent of the solve's previous kernel.  The matrix is fixed
+  // during a solve, so its first rows are staged while that kernel finishes; the vectors and
+  // scalars it wrote are read after it has completed.
+  const int nfirst = ngroups < NS ? ngroups : NS;
+  if (producer) {
+    for (int g = 0; g < nfirst; ++g) {
+      uintptr_t a0 = 0;
+      const uint32_t bytes = source(g, a0);
+      uint32_t total = matrix ? bytes : 0u;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+      if (plane_lane == 0) mbar_more_tx(smem_addr(&full[g]), total);
+      __syncwarp();
+      issue(g, matrix, a0, bytes);
+    }
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   Scal *sc = a.sc;
   if (KIND == K3 && a.in_loop && blockIdx.x == 0 && t == 0) {
@@ -507,28 +612,21 @@ __global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const 
     const unsigned int b = ++sc->body;
     if (sc->done || sc->fault || b > (unsigned int)sc->hc_max + 8u) cudaGraphSetConditional(a.loop, 0u);
   }
-  if (sc->done || sc->fault) return;
+  if (sc->done || sc->fault) {
+    // let the copies in flight land before the block leaves
+    if (producer && plane_lane == 0)
+      for (int g = 0; g < nfirst; ++g) {
+        mbar_arrive(smem_addr(&full[g]));
+        mbar_wait(smem_addr(&full[g]), 0u, kWaitLimit);
+      }
+    return;
+  }
   const int wait_limit = sc->wait_limit;
-  __syncthreads();
 
   double acc0 = 0.0, acc1 = 0.0;
+  double omega = 0.0;                 // K3: of this iteration
   if (producer) {
-    // lane rr*NCP + c owns copy c of row rr of a group: its source address at row ja + rr,
-    // the length and the allocation end; the first element of that copy inside its staged
-    // segment goes to off[stage][rr][c] for the consumers
-    const int lane = t - SX;
-    const int lrow = lane / NCP, lcopy = lane % NCP;
-    uintptr_t c_addr = 0, c_cap = 0;
-    uint32_t c_len = 0;
-    if (lane < RS * NCP) {
-      const T *base, *lim;
-      int dj, di, n;
-      copy_desc<T, KIND>(a, nc, lcopy, base, dj, di, n, lim);
-      c_addr = (uintptr_t)(base + ((long long)(ja + lrow + dj) * ix + i0 + di));
-      c_len = (uint32_t)(n * sizeof(T));
-      c_cap = (uintptr_t)lim & ~(uintptr_t)15;
-    }
-    const uintptr_t row_bytes = (uintptr_t)ix * sizeof(T);
+    const int lane = plane_lane;
     int issued = 0;
     for (int g = 0; g < ngroups; ++g) {
       const int st = g % NS;
@@ -541,35 +639,27 @@ __global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const 
         }
       }
       uintptr_t a0 = 0;
-      uint32_t bytes = 0;
-      if (lane < RS * NCP && g * RS + lrow < nrows) {
-        const uintptr_t ad = c_addr + (uintptr_t)(g * RS) * row_bytes;
-        a0 = ad & ~(uintptr_t)15;
-        uintptr_t end = (ad + c_len + 15) & ~(uintptr_t)15;
-        if (end > c_cap) end = c_cap;
-        bytes = (uint32_t)(end - a0);
-        if (!UNI) off[st][lrow][lcopy] = (int)((ad - a0) / sizeof(T));
-      }
-      uint32_t total = bytes;
+      const uint32_t bytes = source(g, a0);
+      const bool mine = owns && (g >= NS || !matrix);       // the first groups' matrix is under way
+      uint32_t total = mine ? bytes : 0u;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-      const uint32_t fb = smem_addr(&full[st]);
       __syncwarp();                               // every lane's off[st] before the arrival
-      if (lane == 0) mbar_expect_tx(fb, total);   // releases off[st] to the consumers
+      if (lane == 0) mbar_expect_tx(smem_addr(&full[st]), total);   // releases off[st]
       __syncwarp();
-      if (bytes)
-        bulk_load(smem_addr(buf + ((size_t)(st * RS + lrow) * NCP + lcopy) * SLOT),
-                  (const void *)a0, bytes, fb);
+      issue(g, mine, a0, bytes);
       issued = g + 1;
     }
     // let every copy in flight land before the block can leave (the consumers have waited
-    // for all of them on the normal path; after a fault some were never waited for)
+    // for all of them on the normal path; after a fault some were never waited for); the first
+    // groups, whose matrix rows were staged above, have all been issued
     if (lane == 0)
       for (int g = issued - NS > 0 ? issued - NS : 0; g < issued; ++g)
         mbar_wait(smem_addr(&full[g % NS]), (uint32_t)((g / NS) & 1), kWaitLimit);
     __syncwarp();
   } else {
-    // scalars of the update formed at each point
+    // scalars of the update formed at each point; alpha and omega from the previous kernel's
+    // block sums, summed here by every block while its first rows are in flight
     T s1 = T(0), s2 = T(0);
     bool first = false;
     if (KIND == K1) {
@@ -577,10 +667,26 @@ __global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const 
       s1 = (T)sc->beta;
       s2 = (T)sc->omega;
     } else if (KIND == K2) {
-      s1 = (T)sc->alpha;
+      double tot[2];
+      sum_parts<SX>(a.part, tot);
+      const double alpha = tot[0] / tot[1];
+      s1 = (T)alpha;
+      if (blockIdx.x == 0 && t == 0) {
+        sc->alphau = tot[0];
+        sc->alphad = tot[1];
+        sc->alpha = alpha;
+      }
     } else if (KIND == K3) {
+      double tot[2];
+      sum_parts<SX>(a.part, tot);
+      omega = tot[0] / tot[1];
       s1 = (T)sc->alpha;
-      s2 = (T)sc->omega;
+      s2 = (T)omega;
+      if (blockIdx.x == 0 && t == 0) {
+        sc->omegau = tot[0];
+        sc->omegad = tot[1];
+        sc->omega = omega;
+      }
     }
     auto form = [&](const T (&v)[3]) -> T {
       if (KIND == KINIT) return v[0];
@@ -743,26 +849,24 @@ __global__ void __launch_bounds__(kBlock, blocks_per_sm<T>()) bicg_kernel(const 
     if (t == 0) atomicExch(&sc->fault, 1);
     return;
   }
+  // K1's and K2's sums are left to the kernel that needs them; KINIT's and K3's, which decide
+  // whether the solve goes on, are made by the last block to finish
+  if (KIND == K1 || KIND == K2) {
+    block_parts<kBlock>(acc0, acc1, a.part_out);
+    return;
+  }
   double tot[2];
-  if (reduce2<kBlock, SX>(acc0, acc1, a.part, &sc->blocks_done, tot)) {
+  if (reduce2<kBlock, SX>(acc0, acc1, a.part_out, &sc->blocks_done, tot)) {
     if (KIND == KINIT) {
       sc->rr = tot[0];
       sc->bb = tot[1];
       sc->count = 0;
       sc->relres = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
       sc->done = !(sc->relres > sc->tol && sc->count <= sc->hc_max);
-    } else if (KIND == K1) {
-      sc->alphau = tot[0];
-      sc->alphad = tot[1];
-      sc->alpha = tot[0] / tot[1];
-    } else if (KIND == K2) {
-      sc->omegau = tot[0];
-      sc->omegad = tot[1];
-      sc->omega = tot[0] / tot[1];
     } else {
       sc->betau = tot[0];
       sc->rr = tot[1];
-      sc->beta = tot[0] / sc->alphau * sc->alpha / sc->omega;
+      sc->beta = tot[0] / sc->alphau * sc->alpha / omega;
       sc->count = sc->count + 1;
       sc->relres = sqrt(tot[1] / sc->bb);
       sc->done = !(sc->relres > sc->tol && sc->count <= sc->hc_max);
@@ -848,6 +952,10 @@ template <typename T, int KIND>
 void launch(const Grid &g, const KParams &k, BicgArgs<T> a, cudaStream_t s) {
   a.ncb = g.ncb;
   a.nrb = g.nrb;
+  // two sets of block sums: K2 reads what K1 left and writes the other set, which K3 reads
+  double *sets[2] = {a.part_out, a.part_out + 2 * (size_t)g.nb};
+  a.part_out = sets[KIND == K2 ? 1 : 0];
+  a.part = sets[KIND == K3 ? 1 : 0];
   // programmatic dependent launch: the kernel's set-up overlaps the previous kernel's tail
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)g.nb, 1, 1);
@@ -877,7 +985,7 @@ BicgArgs<T> make_args(const T *m, const T *g, std::initializer_list<const T *> w
   for (const T *v : o) a.o[n++] = v;
   n = 0;
   for (T *v : out) a.out[n++] = v;
-  a.part = part;
+  a.part_out = part;
   a.sc = sc;
   return a;
 }
@@ -975,7 +1083,7 @@ cudaError_t hc_create(const KParams &k, bool mixed, HcEngine **out) {
       mf(&e->x32[h], fv); mf(&e->p32[h], fv); mf(&e->ap32[h], fv);
     }
   }
-  md(&e->part, sizeof(double) * 2 * (size_t)std::max(e->grid64.nb, e->grid32.nb));
+  md(&e->part, sizeof(double) * 4 * (size_t)std::max(e->grid64.nb, e->grid32.nb));
   if (err == cudaSuccess) err = cudaMalloc(&e->sc, sizeof(hc::Scal));
   if (err == cudaSuccess) err = cudaMemset(e->sc, 0, sizeof(hc::Scal));
   if (err == cudaSuccess) err = cudaMalloc(&e->sc32, sizeof(hc::Scal));
