@@ -51,7 +51,7 @@ template <> struct Tile<1, 0> {
   static constexpr int TX = 128, TY = 1, NT = 128, MINB = 4, NI = NT;
 };
 template <> struct Tile<2, 1> {
-  static constexpr int TX = 8, TY = 4, NT = 192, MINB = 2, NI = 96;
+  static constexpr int TX = 8, TY = 4, NT = 192, MINB = 2, NI = 96;   // + a control warp
 };
 template <> struct Tile<1, 1> {
   static constexpr int TX = 31, TY = 1, NT = 64, MINB = 4, NI = 32;
@@ -386,34 +386,51 @@ __device__ __forceinline__ void store_cell(double *U, const KParams &p, int gi, 
   if (near_boundary<NDIM>(p, gi, gj)) write_ghosts<NDIM, NVM + 5, true>(p, gi, gj, U, v);
 }
 
-// Block-wide min/max into the reduction slots (one atomic per block).
-template <int NT>
+// Maximum and minimum over a warp of the bits of doubles that are positive or +0 (they order
+// like the doubles), a 32-bit half at a time.
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
+  const unsigned h = (unsigned)(v >> 32), m = __reduce_max_sync(0xffffffffu, h);
+  const unsigned l = __reduce_max_sync(0xffffffffu, h == m ? (unsigned)v : 0u);
+  return (unsigned long long)m << 32 | l;
+}
+__device__ __forceinline__ unsigned long long warp_min_bits(unsigned long long v) {
+  const unsigned h = (unsigned)(v >> 32), m = __reduce_min_sync(0xffffffffu, h);
+  const unsigned l = __reduce_min_sync(0xffffffffu, h == m ? (unsigned)v : 0xffffffffu);
+  return (unsigned long long)m << 32 | l;
+}
+
+// Block-wide min/max into the reduction slots (one atomic per block).  dtc counts below 10
+// (cfl_mhd's start), rho and gr above 0; NaN counts as these.  ONE: the values are all in the
+// first warp.
+template <int NT, bool ONE = false>
 __device__ __forceinline__ void block_reduce_cfl(double dtc, double rho, double gr, DevCtrl *ctrl,
                                                  int slot) {
-  __shared__ double s_red[3][NT / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
-    rho = fmax(rho, __shfl_xor_sync(0xffffffffu, rho, o));
-    gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
-  }
+  unsigned long long d = dbits(dtc < 10.0 ? dtc : 10.0), r = dbits(rho > 0.0 ? rho : 0.0),
+                     g = dbits(gr > 0.0 ? gr : 0.0);
   const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-  if (l == 0) {
-    s_red[0][w] = dtc;
-    s_red[1][w] = rho;
-    s_red[2][w] = gr;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < NT / 32; ++k) {
-      dtc = fmin(dtc, s_red[0][k]);
-      rho = fmax(rho, s_red[1][k]);
-      gr = fmax(gr, s_red[2][k]);
+  if (ONE && w > 0) return;
+  d = warp_min_bits(d);
+  r = warp_max_bits(r);
+  g = warp_max_bits(g);
+  if (!ONE) {
+    __shared__ unsigned long long s_red[3][NT / 32];
+    if (l == 0) {
+      s_red[0][w] = d;
+      s_red[1][w] = r;
+      s_red[2][w] = g;
     }
-    // all values are positive (or +0), so the bit patterns order like the doubles
-    atomicMin(&ctrl->red_dt[slot], dbits(dtc));
-    atomicMax(&ctrl->red_rho[slot], dbits(rho));
-    atomicMax(&ctrl->red_gr[slot], dbits(gr));
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 1; k < NT / 32; ++k) {
+        d = min(d, s_red[0][k]);
+        r = max(r, s_red[1][k]);
+        g = max(g, s_red[2][k]);
+      }
+  }
+  if (threadIdx.x == 0) {
+    atomicMin(&ctrl->red_dt[slot], d);
+    atomicMax(&ctrl->red_rho[slot], r);
+    atomicMax(&ctrl->red_gr[slot], g);
   }
 }
 
@@ -564,13 +581,20 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Threads of a CTA: the small tiles (S = 1) have one warp more, which reads the control block and
+// forms dt while the others convert the tile.
+template <int NDIM, int S>
+constexpr int tile_threads() {
+  return Tile<NDIM, S>::NT + (S == 1 ? 32 : 0);
+}
+
 template <int NDIM, int NVM, int STAGE, int X, int S>
-__global__ void __launch_bounds__(Tile<NDIM, S>::NT, Tile<NDIM, S>::MINB)
+__global__ void __launch_bounds__(tile_threads<NDIM, S>(), Tile<NDIM, S>::MINB)
 stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, const double *U0,
              double *Uo, DevCtrl *ctrl, int dt_mode, int epi,
              const __grid_constant__ CUtensorMap tmap, int use_tma, int rows) {
   constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = Tile<NDIM, S>::NT;
-  constexpr int NI = Tile<NDIM, S>::NI;
+  constexpr int NI = Tile<NDIM, S>::NI, NTA = tile_threads<NDIM, S>();
   constexpr int NV = NVM + 5;
   constexpr int RX = TX + 2 * kH, RY = NDIM == 2 ? TY + 2 * kH : 1, RR = RX * RY;
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
@@ -581,6 +605,8 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   double *sFy = sFx + NV * NFX;
   constexpr bool COL = (X & 1) != 0, RES = (X & 2) != 0;
   double *sE = sFy + NV * NFY;  // RES only: E of the tile's cells and one ring
+  // S = 1: U0 and the updated state of the tile's cells (one warp's)
+  double *sU0 = sE + (RES ? 3 * EN : 0), *sN = sU0 + NV * 32;
   __shared__ double s_dt, s_cmax;
   __shared__ int s_exit, s_epi, s_slot;
   __shared__ __align__(8) unsigned long long s_bar;
@@ -595,18 +621,31 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   const int i0 = p.m0 + blockIdx.x * TX;
   const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
   const bool staged = NDIM == 2 && use_tma && (tma_smem_addr(sV) & 127u) == 0;
-  if (tid == 0 && staged) tma_bar_init(&s_bar);
+  const bool control = tid == (S == 1 ? NT : 0);
+  if (control && staged) {
+    tma_bar_init(&s_bar);
+    tma_prefetch_map(&tmap);
+  }
   // Launched as a programmatic dependent of the previous kernel on the stream: it may start
   // while that one finishes, and reads nothing that one wrote before this wait.
   pdl_wait();
   pdl_launch_dependents();
-  if (tid == 0) {
-    if (staged) {
-      // all planes of the tile and its halo by one TMA load into sV (cells outside the array
-      // read as zero), in flight while the control block is read
-      tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
-      tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
+  const long long nc = p.nc;
+  if (control && staged) {
+    // all planes of the tile and its halo by one TMA load into sV (cells outside the array
+    // read as zero), in flight while the control block is read
+    tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
+    tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
+  }
+  if (S == 1) {
+    if (staged) __syncthreads();      // the barrier's initialisation, before anyone waits on it
+    for (int k = tid; k < NV * 32; k += NTA) {
+      const int n = k / 32, c = k % 32, ci = i0 + c % TX, cj = j0 + c / TX;
+      if (c < TX * TY && ci < p.m0 + p.nx && (NDIM == 1 || cj < p.m1 + p.ny))
+        cp_async8(sU0 + k, U0 + n * nc + (long long)cj * p.ix + ci);
     }
+  }
+  auto read_control = [&]() {
     // the control block by independent loads (one round trip), then dt
     double dt, cmax;
     if (STAGE == 1) {
@@ -631,63 +670,13 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     }
     s_dt = dt;
     s_cmax = cmax;
-  }
-  __syncthreads();
-  if (s_exit) {
-    if (STAGE == 1 && block0 && tid == 0) {
-      if (ctrl->nan_flag && ctrl->status == 0) ctrl->status = 3;  // PIP_ERR_NAN
-      ctrl->done = 1;
-      ctrl->skip = 1;
-    }
-    if (staged) tma_bar_wait(&s_bar, kTmaWaitLimit);   // no copy in flight when the CTA leaves
-    return;
-  }
-  const double dt = s_dt, cmax = s_cmax;
-  if (STAGE == 1 && block0 && tid == 0) {
-    ctrl->skip = 0;
-    ctrl->floored = 0;
-    if (dt_mode == 1) {
-      // loop bookkeeping of main.f90:31,58 for this step (no block of stage 1 reads these)
-      const long long st = ctrl->step;
-      ctrl->dt = dt;
-      ctrl->cmax = cmax;
-      const double tn = ctrl->time + dt;
-      ctrl->time_next = tn;
-      ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
-                    (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
-      const int ns = (int)((st + 1) & 1);
-      ctrl->slot = ns;
-      ctrl->red_dt[ns] = dbits(fmin(10.0, p.resi_dt));  // cfl_mhd's start, cfl_resi's bound
-      ctrl->red_rho[ns] = 0ull;
-      ctrl->red_gr[ns] = 0ull;
-      ctrl->red_ip[ns] = 0ull;
-      ctrl->red_nx[ns] = 0ull;
-    }
-  }
-  if (STAGE == 2 && dt_mode == 1 && !(RES && p.resi == 2) && block0 && tid == 0) {
-    // end of step: time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636); no
-    // block of stage 2 reads what changes here
-    ctrl->time = ctrl->time_next;
-    ctrl->step = ctrl->step + 1;
-    if (ctrl->last) ctrl->done = 1;
-    if (dt <= 1.0e-12) {
-      ctrl->done = 1;
-      if (ctrl->status == 0) ctrl->status = 4;  // PIP_ERR_DT
-    }
-  }
-
-  if (STAGE == 1 && RES && p.resi == 2 && block0 && tid == 0) {
-    // stage 2 takes the minimum of cfl_resi's bound into this word; no kernel reads it
-    // between the stages
-    *p.resi_bound = dbits(INFINITY);
-  }
-
+  };
   const double gm = p.gm, ro_lim = p.ro_lim, pr_lim = p.pr_lim;
-  const long long nc = p.nc;
 
   // ---- 1. stage state of the tile and its halo -> primitives in shared memory
   // Each cell's conversion is one thread's (both species); with S = 1 and no energy rewrite
   // a unit is one species of a cell.  The TMA's tile is converted in place.
+  auto convert_tile = [&]() {
   if (staged && !tma_bar_wait(&s_bar, kTmaWaitLimit)) {
     // the tile did not arrive: flag the stage (the run stops with PIP_ERR_ITER; this
     // tile's results are void) and let the copy land (bounded) before going on, so that
@@ -737,14 +726,80 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     if (NDIM == 2 && staged) convert(sV + idx, RR, idx, ions, neutrals);
     else convert(Us + (long long)gj * p.ix + gi, nc, idx, ions, neutrals);
   }
-  __syncthreads();
+  };
+  if (S == 0) {
+    if (control) read_control();
+    __syncthreads();
+  } else {
+    if (tid >= NT) {
+      if (control) read_control();
+    } else {
+      convert_tile();
+    }
+    __syncthreads();
+  }
+  if (s_exit) {
+    if (STAGE == 1 && block0 && control) {
+      if (ctrl->nan_flag && ctrl->status == 0) ctrl->status = 3;  // PIP_ERR_NAN
+      ctrl->done = 1;
+      ctrl->skip = 1;
+    }
+    // no copy in flight when the CTA leaves
+    if (staged) tma_bar_wait(&s_bar, kTmaWaitLimit);
+    if (S == 1) cp_async_wait();
+    return;
+  }
+  const double dt = s_dt, cmax = s_cmax;
+  if (STAGE == 1 && block0 && control) {
+    ctrl->skip = 0;
+    ctrl->floored = 0;
+    if (dt_mode == 1) {
+      // loop bookkeeping of main.f90:31,58 for this step (no block of stage 1 reads these)
+      const long long st = ctrl->step;
+      ctrl->dt = dt;
+      ctrl->cmax = cmax;
+      const double tn = ctrl->time + dt;
+      ctrl->time_next = tn;
+      ctrl->last = ((ctrl->t_end > 0.0 && tn >= ctrl->t_end) ||
+                    (ctrl->nsteps > 0 && st + 1 >= ctrl->nsteps)) ? 1 : 0;
+      const int ns = (int)((st + 1) & 1);
+      ctrl->slot = ns;
+      ctrl->red_dt[ns] = dbits(fmin(10.0, p.resi_dt));  // cfl_mhd's start, cfl_resi's bound
+      ctrl->red_rho[ns] = 0ull;
+      ctrl->red_gr[ns] = 0ull;
+      ctrl->red_ip[ns] = 0ull;
+      ctrl->red_nx[ns] = 0ull;
+    }
+  }
+  if (STAGE == 2 && dt_mode == 1 && !(RES && p.resi == 2) && block0 && control) {
+    // end of step: time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636); no
+    // block of stage 2 reads what changes here
+    ctrl->time = ctrl->time_next;
+    ctrl->step = ctrl->step + 1;
+    if (ctrl->last) ctrl->done = 1;
+    if (dt <= 1.0e-12) {
+      ctrl->done = 1;
+      if (ctrl->status == 0) ctrl->status = 4;  // PIP_ERR_DT
+    }
+  }
+
+  if (STAGE == 1 && RES && p.resi == 2 && block0 && control) {
+    // stage 2 takes the minimum of cfl_resi's bound into this word; no kernel reads it
+    // between the stages
+    *p.resi_bound = dbits(INFINITY);
+  }
+
+  if (S == 0) {
+    convert_tile();
+    __syncthreads();
+  }
   // resi 2, stage 2: cfl_resi's bound over this tile's interior cells with the eta of this
   // stage (the last set_resistivity before the next cfl)
   double rb = INFINITY;
   if (RES) {
     // E = eta*curl B once per cell of the tile and its first ring (each enters four faces)
     const int iend_ = p.m0 + p.nx, jend_ = NDIM == 2 ? p.m1 + p.ny : 1;
-    for (int idx = tid; idx < EN; idx += NT) {
+    for (int idx = tid; idx < EN; idx += NTA) {
       const int er = idx % EW, ej = idx / EW;
       const int gi = i0 - 1 + er, gj = NDIM == 2 ? j0 - 1 + ej : 0;
       if (gi > p.ix - 2 || (NDIM == 2 && gj > p.jx - 2)) continue;
@@ -760,7 +815,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
         rb = fmin(rb, p.safety * (gmin * gmin) / fmax(eta, 1.0e-8));
       }
     }
-    if (STAGE == 2 && p.resi == 2) block_min_to<NT>(rb, p.resi_bound);
+    if (STAGE == 2 && p.resi == 2) block_min_to<NTA>(rb, p.resi_bound);
     __syncthreads();
   }
 
@@ -771,7 +826,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 
   // ---- 2. face fluxes (set_flux): x faces then y faces of the tile
   const bool ion_faces = S == 0 || tid < NI, neutral_faces = S == 0 || tid >= NI;
-  const int f0 = S == 1 && tid >= NI ? tid - NI : tid;
+  const int f0 = S == 0 || tid < NI ? tid : tid < NT ? tid - NI : NFX + NFY;
   for (int f = f0; f < NFX + NFY; f += NI) {
     int a, s, perm_y;
     double *Fout;
@@ -865,16 +920,27 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
                  sE[2 * EN + e1], bx[a], bx[a1], by[a], by[a1], bz[a], bz[a1]);
     }
   }
+  if (S == 1) cp_async_wait();
   __syncthreads();
 
   // ---- 3. per-cell source, update, epilogue
   double dtc = 10.0, rhoc = 0.0, grc = 0.0;
+  // S = 1: the ghost images of a boundary tile are written by all warps, some planes each
+  const bool edge = S == 1 && (i0 < 2 * p.m0 || i0 + TX > p.ix - 2 * p.m0 ||
+                               (NDIM == 2 && (j0 < 2 * p.m1 || j0 + TY > p.jx - 2 * p.m1)));
   if (valid) {
     const long long q = (long long)gj * p.ix + gi;
     const double dt_sub = STAGE == 1 ? dt / 2.0 : dt / 1.0;  // dt/(t_order-istep+1)
     const double dt_coll = dt * 0.5;                          // set_dt_coll, t_order=2
     double a_m[NVM], a_h[5];  // U0 of the cell
-    load_cell<NVM>(U0, q, nc, a_m, a_h);
+    if (S == 1) {
+#pragma unroll
+      for (int n = 0; n < NVM; ++n) a_m[n] = sU0[n * 32 + tid];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) a_h[n] = sU0[(NVM + n) * 32 + tid];
+    } else {
+      load_cell<NVM>(U0, q, nc, a_m, a_h);
+    }
     double ac_s = p.ac;       // alpha_c of the stage
     double S_m[5], S_h[5];
     Prim<double> qm, qh;      // primitives of the stage state as source_PIP's cq2pv leaves them
@@ -1108,7 +1174,16 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     for (int n = 0; n < 5; ++n) top = max(top, __double2hiint(n_h[n]) & 0x7fffffff);
     const bool bad = top >= 0x7ff00000;
     if (bad) atomicOr(&ctrl->nan_flag, 1);
-    store_cell<NDIM, NVM>(Uo, p, gi, gj, n_m, n_h);
+    if (S == 1) {
+#pragma unroll
+      for (int n = 0; n < NV; ++n) {
+        const double v = n < NVM ? n_m[n] : n_h[n - NVM];
+        Uo[q + n * nc] = v;
+        if (edge) sN[n * 32 + tid] = v;
+      }
+    } else {
+      store_cell<NDIM, NVM>(Uo, p, gi, gj, n_m, n_h);
+    }
     if (STAGE == 2 && COL && p.col_type) {
       // the alpha_c field that the next cfl reads (cfl_pn_col, Scheme_rot.f90:305-313)
       p.acf[q] = ac_s;
@@ -1118,10 +1193,22 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       }
     }
   }
-  if (STAGE == 2 && COL && p.col_type) exchanged_ghost_ac<NDIM, NVM, TX, TY, NT>(p, Us, i0, j0, tid, by, nby);
+  if (STAGE == 2 && COL && p.col_type) exchanged_ghost_ac<NDIM, NVM, TX, TY, NTA>(p, Us, i0, j0, tid, by, nby);
   if (STAGE == 2 && s_epi == 2) {
     if (RES && p.resi == 2) dtc = fmin(dtc, rb);  // the next step's cfl_resi
-    block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, s_slot);
+    block_reduce_cfl<NTA, S == 1>(dtc, rhoc, grc, ctrl, s_slot);
+  }
+  if (S == 1 && edge) {
+    __syncthreads();
+    const int c = tid % 32, ci = i0 + c % TX, cj = j0 + c / TX;
+    if (c < TX * TY && ci < iend && (NDIM == 1 || cj < jend) && near_boundary<NDIM>(p, ci, cj))
+      ghost_images<NDIM>(p, ci, cj, [&](long long g, unsigned flips) {
+#pragma unroll
+        for (int k = 0; k < (NV + NTA / 32 - 1) / (NTA / 32); ++k) {
+          const int n = tid / 32 + k * (NTA / 32);
+          if (n < NV) Uo[g + n * nc] = flipped(sN[n * 32 + c], flips, n);
+        }
+      });
   }
   if (STAGE == 2 && RES && dt_mode == 1 && p.resi == 2) {
     // end of step, by the last block to finish: the time increment needs every block's bound
@@ -1451,7 +1538,8 @@ constexpr size_t stage_smem_bytes() {
   constexpr int RR = (TX + 2 * kH) * (NDIM == 2 ? TY + 2 * kH : 1);
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
   constexpr int EN = (TX + 2) * (NDIM == 2 ? TY + 2 : 1);
-  return sizeof(double) * ((NVM + 5) * (RR + NFX + NFY) + ((X & 2) ? 3 * EN : 0));
+  return sizeof(double) * ((NVM + 5) * (RR + NFX + NFY) + ((X & 2) ? 3 * EN : 0) +
+                           (S == 1 ? 2 * (NVM + 5) * 32 : 0));
 }
 
 template <int NDIM, int NVM, int STAGE, int X>
@@ -1512,7 +1600,7 @@ template <int NDIM, int NVM, int STAGE, int X, int S>
 static cudaError_t launch_tiles(const KParams &p, const double *Us, const double *U0, double *Uo,
                                 DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                 const CUtensorMap *tm, int rows) {
-  constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = Tile<NDIM, S>::NT;
+  constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = tile_threads<NDIM, S>();
   const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
   if (NDIM == 1) rows = 0;
   const int gy = rows == 0 ? nby : rows == 1 ? (nby < 2 ? nby : 2) : nby - 2;

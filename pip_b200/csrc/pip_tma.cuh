@@ -38,6 +38,17 @@ __device__ __forceinline__ void tma_bar_expect(unsigned long long *bar, uint32_t
                : "memory");
 }
 
+// Fetches the map's descriptor ahead of its first use.
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)map) : "memory");
+}
+
+// An 8-byte copy from global to shared memory, waited for by cp_async_wait of the same thread.
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tma_smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // One 3D tile (x0, y0, plane 0) of the map into dst; completes on bar.
 __device__ __forceinline__ void tma_load_tile(void *dst, const CUtensorMap *map, int x0, int y0,
                                               unsigned long long *bar) {
