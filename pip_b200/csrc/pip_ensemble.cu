@@ -323,10 +323,7 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
           grc = fmax(grc, fmax(g1, g2));
         }
       }
-#pragma unroll
-      for (int n = 0; n < NVM; ++n) bad |= !isfinite(n_m[n]);
-#pragma unroll
-      for (int n = 0; n < 5; ++n) bad |= !isfinite(n_h[n]);
+      bad |= mixed::not_finite(n_m) || mixed::not_finite(n_h);
       double u[NV];
 #pragma unroll
       for (int n = 0; n < NV; ++n) {

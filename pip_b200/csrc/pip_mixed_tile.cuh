@@ -131,10 +131,9 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
         const float *vp = sV + (NVM - 1) * RR + a;
         const double b0 = vb[-s], b1 = vb[0], b2 = vb[s], b3 = vb[2 * s];
         const double p0 = vp[-s], p1 = vp[0], p2 = vp[s], p3 = vp[2 * s];
-        const double bl = b1 + 0.5 * minmod<double>(b0, b1, b2);
-        const double br = b2 - 0.5 * minmod<double>(b1, b2, b3);
-        const double pl = p1 + 0.5 * minmod<double>(p0, p1, p2);
-        const double pr = p2 - 0.5 * minmod<double>(p1, p2, p3);
+        double bl, br, pl, pr;
+        face_pair(b0, b1, b2, b3, bl, br);
+        face_pair(p0, p1, p2, p3, pl, pr);
         const double ch = cmax;
         sD6[f] = 0.5 * (pl + pr - ch * (br - bl));
         sD9[f] = 0.5 * (ch * ch * (bl + br) - ch * (pr - pl));
@@ -284,10 +283,7 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
         grc = fmax(grc, fmax(g1, g2));
       }
     }
-#pragma unroll
-    for (int n = 0; n < NVM; ++n) bad |= !isfinite(n_m[n]);
-#pragma unroll
-    for (int n = 0; n < 5; ++n) bad |= !isfinite(n_h[n]);
+    bad |= not_finite(n_m) || not_finite(n_h);
     double u[NV];
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
