@@ -449,11 +449,19 @@ __device__ __forceinline__ void cell_e(const double *bx, const double *by, const
                                        double &ez, double &eta) {
   double r1 = 0.0, r2, r3;
 #if PIP_RCP
-  // the FMA build multiplies by 1/(2 dx), 1/(2 dy)
+  // the FMA builds multiply by 1/(2 dx), 1/(2 dy)
+#if PIP_FAST
+  const double rx = 0.5 * rcp_(p.dx[gi]);
+#else
   const double rx = 1.0 / (2.0 * p.dx[gi]);
+#endif
   r2 = -((bz[c + 1] - bz[c - 1]) * rx);
   if (NDIM == 2) {
+#if PIP_FAST
+    const double ry = 0.5 * rcp_(p.dy[gj]);
+#else
     const double ry = 1.0 / (2.0 * p.dy[gj]);
+#endif
     r1 = (bz[c + sy] - bz[c - sy]) * ry;
     r3 = (by[c + 1] - by[c - 1]) * rx - (bx[c + sy] - bx[c - sy]) * ry;
   } else {
@@ -588,6 +596,16 @@ constexpr int tile_threads() {
   return Tile<NDIM, S>::NT + (S == 1 ? 32 : 0);
 }
 
+// Columns that a staged tile has more on each side than its halo: with resistivity the margin is
+// 3, a tile's halo starts at an odd column, and the TMA copies from 16-byte boundaries, i.e.
+// one FP64 column earlier.  A step of 500x300 cells with resistivity: 71.1 us with the tile read
+// by each thread's loads (46 % of the issue slots used, the rest waits of the loads and barriers
+// before the conversion), 65.0 us with the wider tile by TMA.
+template <int NDIM, int X>
+constexpr int tile_xo() {
+  return NDIM == 2 && (X & 2) ? 1 : 0;
+}
+
 template <int NDIM, int NVM, int STAGE, int X, int S>
 __global__ void __launch_bounds__(tile_threads<NDIM, S>(), Tile<NDIM, S>::MINB)
 stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, const double *U0,
@@ -596,15 +614,17 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = Tile<NDIM, S>::NT;
   constexpr int NI = Tile<NDIM, S>::NI, NTA = tile_threads<NDIM, S>();
   constexpr int NV = NVM + 5;
-  constexpr int RX = TX + 2 * kH, RY = NDIM == 2 ? TY + 2 * kH : 1, RR = RX * RY;
+  constexpr int XO = tile_xo<NDIM, X>();
+  constexpr int RX = TX + 2 * kH + 2 * XO, RY = NDIM == 2 ? TY + 2 * kH : 1, RR = RX * RY;
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
   constexpr int EW = TX + 2, EH = NDIM == 2 ? TY + 2 : 1, EN = EW * EH;
   extern __shared__ __align__(128) double smem[];
   double *sV = smem;                 // first: the TMA destination (128-byte aligned)
-  double *sFx = sV + NV * RR;
-  double *sFy = sFx + NV * NFX;
+  // fluxes: plane n of x face f at sF[n*NF + f], of y face g at sF[n*NF + NFX + g]
+  constexpr int NF = NFX + NFY;
+  double *sF = sV + NV * RR;
   constexpr bool COL = (X & 1) != 0, RES = (X & 2) != 0;
-  double *sE = sFy + NV * NFY;  // RES only: E of the tile's cells and one ring
+  double *sE = sF + NV * NF;  // RES only: E of the tile's cells and one ring
   // S = 1: U0 and the updated state of the tile's cells (one warp's)
   double *sU0 = sE + (RES ? 3 * EN : 0), *sN = sU0 + NV * 32;
   __shared__ double s_dt, s_cmax;
@@ -635,7 +655,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     // all planes of the tile and its halo by one TMA load into sV (cells outside the array
     // read as zero), in flight while the control block is read
     tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
-    tma_load_tile(sV, &tmap, i0 - kH, j0 - kH, &s_bar);
+    tma_load_tile(sV, &tmap, i0 - kH - XO, j0 - kH, &s_bar);
   }
   if (S == 1) {
     if (staged) __syncthreads();      // the barrier's initialisation, before anyone waits on it
@@ -717,7 +737,8 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   for (int u = tid; u < (SPLITP ? 2 : 1) * RR; u += NT) {
     const int idx = SPLITP && u >= RR ? u - RR : u;
     const bool ions = !SPLITP || u < RR, neutrals = !SPLITP || u >= RR;
-    const int ri = idx % RX, rj = idx / RX;
+    const int ri = idx % RX - XO, rj = idx / RX;
+    if (XO && (ri < 0 || ri >= TX + 2 * kH)) continue;
     // the corners only for the curl of B next to the tile's corner faces (resistivity)
     if (NDIM == 2 && !RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH))
       continue;
@@ -803,7 +824,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       const int er = idx % EW, ej = idx / EW;
       const int gi = i0 - 1 + er, gj = NDIM == 2 ? j0 - 1 + ej : 0;
       if (gi > p.ix - 2 || (NDIM == 2 && gj > p.jx - 2)) continue;
-      const int c = (NDIM == 2 ? (ej + kH - 1) * RX : 0) + er + kH - 1;
+      const int c = (NDIM == 2 ? (ej + kH - 1) * RX : 0) + er + kH - 1 + XO;
       double ex, ey, ez, eta;
       cell_e<NDIM>(sV + 5 * RR, sV + 6 * RR, sV + 7 * RR, sV, c, RX, p, gi, gj, ex, ey, ez, eta);
       sE[idx] = ex;
@@ -829,26 +850,18 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   const int f0 = S == 0 || tid < NI ? tid : tid < NT ? tid - NI : NFX + NFY;
   for (int f = f0; f < NFX + NFY; f += NI) {
     int a, s, perm_y;
-    double *Fout;
-    int fo, nf;
     if (f < NFX) {
       const int fi = f % (TX + 1), fj = f / (TX + 1);
       if (i0 + fi - 1 >= iend || (NDIM == 2 && j0 + fj >= jend)) continue;
-      a = (NDIM == 2 ? (fj + kH) * RX : 0) + fi + kH - 1;  // left cell of the face
+      a = (NDIM == 2 ? (fj + kH) * RX : 0) + fi + kH - 1 + XO;  // left cell of the face
       s = 1;
       perm_y = 0;
-      Fout = sFx;
-      fo = f;
-      nf = NFX;
     } else {
       const int g = f - NFX, fi = g % TX, fj = g / TX;
       if (i0 + fi >= iend || j0 + fj - 1 >= jend) continue;
-      a = (fj + kH - 1) * RX + fi + kH;  // lower cell of the face
+      a = (fj + kH - 1) * RX + fi + kH + XO;  // lower cell of the face
       s = RX;
       perm_y = 1;
-      Fout = sFy;
-      fo = g;
-      nf = NFY;
     }
     if (ion_faces) {
       double vl[NVM], vr[NVM], fx[NVM];
@@ -865,7 +878,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 #pragma unroll
       for (int n = 0; n < NVM; ++n) {
         const int dst = perm_y ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
-        Fout[dst * nf + fo] = fx[n];
+        sF[dst * NF + f] = fx[n];
       }
     }
     if (neutral_faces) {
@@ -882,7 +895,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 #pragma unroll
       for (int n = 0; n < 5; ++n) {
         const int dst = perm_y ? (n == 1 ? 2 : n == 2 ? 1 : n) : n;
-        Fout[(NVM + dst) * nf + fo] = fx[n];
+        sF[(NVM + dst) * NF + f] = fx[n];
       }
     }
   }
@@ -890,33 +903,26 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     // resistive_flux's terms, added by the thread that wrote the face's flux (same faces
     // per thread as above), in a loop of their own to keep the Riemann solvers' registers
     for (int f = S == 1 && tid >= NI ? NFX + NFY : tid; f < NFX + NFY; f += NI) {
-      int a, s, nf, fo, e0, e1;
-      double *Fout;
+      int a, s, e0, e1;
       const bool ydir = f >= NFX;
       if (!ydir) {
         const int fi = f % (TX + 1), fj = f / (TX + 1);
         if (i0 + fi - 1 >= iend || (NDIM == 2 && j0 + fj >= jend)) continue;
-        a = (NDIM == 2 ? (fj + kH) * RX : 0) + fi + kH - 1;
+        a = (NDIM == 2 ? (fj + kH) * RX : 0) + fi + kH - 1 + XO;
         s = 1;
-        Fout = sFx;
-        fo = f;
-        nf = NFX;
         e0 = (NDIM == 2 ? (fj + 1) * EW : 0) + fi;
         e1 = e0 + 1;
       } else {
         const int g = f - NFX, fi = g % TX, fj = g / TX;
         if (i0 + fi >= iend || j0 + fj - 1 >= jend) continue;
-        a = (fj + kH - 1) * RX + fi + kH;
+        a = (fj + kH - 1) * RX + fi + kH + XO;
         s = RX;
-        Fout = sFy;
-        fo = g;
-        nf = NFY;
         e0 = fj * EW + fi + 1;
         e1 = e0 + EW;
       }
       const int a1 = a + s;
       const double *bx = sV + 5 * RR, *by = sV + 6 * RR, *bz = sV + 7 * RR;
-      face_terms(Fout, nf, fo, ydir, sE[e0], sE[EN + e0], sE[2 * EN + e0], sE[e1], sE[EN + e1],
+      face_terms(sF, NF, f, ydir, sE[e0], sE[EN + e0], sE[2 * EN + e0], sE[e1], sE[EN + e1],
                  sE[2 * EN + e1], bx[a], bx[a1], by[a], by[a1], bz[a], bz[a1]);
     }
   }
@@ -950,7 +956,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       // u2v's, the same up to rounding) and forms the exchange from them, so stage 2 does
       // not read its stage state again; where the density floor acts, u2v's velocity is
       // another one and the state is converted as the reference does.
-      const int c = (NDIM == 2 ? (tj + kH) * RX : 0) + ti + kH;
+      const int c = (NDIM == 2 ? (tj + kH) * RX : 0) + ti + kH + XO;
       qm = Prim<double>{sV[c], sV[RR + c], sV[2 * RR + c], sV[3 * RR + c], sV[4 * RR + c]};
       qh = Prim<double>{sV[NVM * RR + c], sV[(NVM + 1) * RR + c], sV[(NVM + 2) * RR + c],
                         sV[(NVM + 3) * RR + c], sV[(NVM + 4) * RR + c]};
@@ -1091,8 +1097,8 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
       const double u0 = n < NVM ? a_m[n] : a_h[n - NVM];
-      double u = u0 - cx * (sFx[n * NFX + fxl + 1] - sFx[n * NFX + fxl]);
-      if (NDIM == 2) u = u - cy * (sFy[n * NFY + fyl + TX] - sFy[n * NFY + fyl]);
+      double u = u0 - cx * (sF[n * NF + fxl + 1] - sF[n * NF + fxl]);
+      if (NDIM == 2) u = u - cy * (sF[n * NF + NFX + fyl + TX] - sF[n * NF + NFX + fyl]);
       if (n < NVM) {
         u = n < 5 ? u + S_m[n] * dt_sub : u + 0.0;
         n_m[n] = u;
@@ -1535,7 +1541,7 @@ __global__ void nan_kernel(const double *__restrict__ U, long long n, int *flag)
 template <int NDIM, int NVM, int X, int S>
 constexpr size_t stage_smem_bytes() {
   constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY;
-  constexpr int RR = (TX + 2 * kH) * (NDIM == 2 ? TY + 2 * kH : 1);
+  constexpr int RR = (TX + 2 * kH + 2 * tile_xo<NDIM, X>()) * (NDIM == 2 ? TY + 2 * kH : 1);
   constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
   constexpr int EN = (TX + 2) * (NDIM == 2 ? TY + 2 : 1);
   return sizeof(double) * ((NVM + 5) * (RR + NFX + NFY) + ((X & 2) ? 3 * EN : 0) +
@@ -1680,9 +1686,10 @@ static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, c
 
 template <int S>
 static bool tile_map_s(const KParams &p, const double *U, CUtensorMap *map) {
-  constexpr int TX = Tile<2, S>::TX, RX = TX + 2 * kH, RY = Tile<2, S>::TY + 2 * kH;
-  return tma_tile_ok(U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), p.m0 - kH, TX, RX, RY) &&
-         tma_encode(map, U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), RX, RY);
+  constexpr int TX = Tile<2, S>::TX, RY = Tile<2, S>::TY + 2 * kH;
+  const int xo = p.resi ? tile_xo<2, 2>() : 0, rx = TX + 2 * kH + 2 * xo;
+  return tma_tile_ok(U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), p.m0 - kH - xo, TX, rx, RY) &&
+         tma_encode(map, U, p.ix, p.jx, p.nvm + 5, (int)sizeof(double), rx, RY);
 }
 static bool tile_map(const KParams &p, const double *U, CUtensorMap *map) {
   if (p.ndim != 2) return false;
