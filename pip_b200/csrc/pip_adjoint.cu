@@ -792,7 +792,7 @@ int pip_adj_create(const pip_params *p, int64_t max_steps, int checkpoint_every,
   };
   cudaError_t e;
   if ((e = cudaGetDevice(&a->device)) != cudaSuccess) return fail(e);
-  if ((e = a->L->prepare()) != cudaSuccess) return fail(e);
+  if ((e = a->L->prepare(&a->kp)) != cudaSuccess) return fail(e);
   if ((e = pip::adjk::prepare()) != cudaSuccess) return fail(e);
   // the reverse sweep (stream) is the critical path; the recomputation of the next segment
   // (stream2) fills the SMs it leaves idle, so it gets the lower priority

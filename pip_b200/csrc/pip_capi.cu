@@ -682,7 +682,7 @@ int pip_ctx_create(const pip_params *p, pip_ctx **out) {
   };
   cudaError_t e = cudaGetDevice(&c->device);
   if (e != cudaSuccess) return fail(e);
-  if ((e = c->L->prepare()) != cudaSuccess) return fail(e);
+  if ((e = c->L->prepare(&c->kp)) != cudaSuccess) return fail(e);
   if (c->mixed && (e = pip::mixed_prepare()) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   const size_t state = c->plane_bytes() * c->nplanes();

@@ -121,7 +121,7 @@ struct DevCtrl {
 
 // Host launchers (one set per arithmetic flavour).
 struct Launchers {
-  cudaError_t (*prepare)();
+  cudaError_t (*prepare)(const KParams *p);   // null: every grid's instances
   // tm: the TMA map of Us for the 2D tiles (tile_map), or null for per-thread loads.  rows
   // (2D): 0 every tile row; 1 the first and the last tile row (those a y-halo exchange
   // sends); 2 the rows between them.  A stage launched as 1 then 2 equals one launch of 0.

@@ -72,8 +72,8 @@ extern "C" int pip_step_noalloc(const pip_params *p, double *U_dev, double dt, d
       if ((e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch)) != cudaSuccess) return cuda_fail(e);
       if (!ptr) return PIP_ERR_CUDA;
       // both FP64 flavours, so a later call with the other fp_exact also finds its limit set
-      if ((e = pip::launchers_fast().prepare()) != cudaSuccess) return cuda_fail(e);
-      if ((e = pip::launchers_exact().prepare()) != cudaSuccess) return cuda_fail(e);
+      if ((e = pip::launchers_fast().prepare(nullptr)) != cudaSuccess) return cuda_fail(e);
+      if ((e = pip::launchers_exact().prepare(nullptr)) != cudaSuccess) return cuda_fail(e);
       g_scratch_addr[dev] = ptr;
     }
     base = g_scratch_addr[dev];

@@ -657,6 +657,40 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     tma_bar_expect(&s_bar, (uint32_t)(NV * RR * sizeof(double)));
     tma_load_tile(sV, &tmap, i0 - kH - XO, j0 - kH, &s_bar);
   }
+  constexpr bool SPLITP = S == 1 && !COL;
+  // calls f(idx, offset of the cell in a plane, ions, neutrals) for this thread's units of the
+  // tile and its halo: a cell, or with SPLITP one species of a cell
+  auto tile_units = [&](auto &&f) {
+    for (int u = tid; u < (SPLITP ? 2 : 1) * RR; u += NT) {
+      const int idx = SPLITP && u >= RR ? u - RR : u;
+      const int ri = idx % RX - XO, rj = idx / RX;
+      if (XO && (ri < 0 || ri >= TX + 2 * kH)) continue;
+      // the corners only for the curl of B next to the tile's corner faces (resistivity)
+      if (NDIM == 2 && !RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH))
+        continue;
+      const int gi = i0 - kH + ri, gj = NDIM == 2 ? j0 - kH + rj : 0;
+      if (gi >= p.ix || gj >= p.jx) continue;
+      f(idx, (long long)gj * p.ix + gi, !SPLITP || u < RR, !SPLITP || u >= RR);
+    }
+  };
+  // Grids of an odd number of columns, which no TMA map describes: the tile by 8-byte
+  // asynchronous copies, in flight while the control block is read; each thread waits for and
+  // converts its own cells in place.  517x333 with walls 67.6 -> 67.0 us a step, 1023x1001 336 ->
+  // 329 against the cells' loads by the thread that converts them, one cell after the other; with
+  // resistivity those stay (699x699: 217 us, by copies 223).
+  const bool copied = NDIM == 2 && !RES && !staged;
+  if (copied && tid < NT) {
+    tile_units([&](int idx, long long q, bool ions, bool neutrals) {
+      if (ions) {
+#pragma unroll
+        for (int n = 0; n < NVM; ++n) cp_async8(sV + n * RR + idx, Us + q + n * nc);
+      }
+      if (neutrals) {
+#pragma unroll
+        for (int n = NVM; n < NV; ++n) cp_async8(sV + n * RR + idx, Us + q + n * nc);
+      }
+    });
+  }
   if (S == 1) {
     if (staged) __syncthreads();      // the barrier's initialisation, before anyone waits on it
     for (int k = tid; k < NV * 32; k += NTA) {
@@ -705,7 +739,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     ctrl->done = 1;
     tma_bar_wait(&s_bar, kTmaWaitLimit);
   }
-  constexpr bool SPLITP = S == 1 && !COL;
+  if (copied) cp_async_wait();
   auto convert = [&](const double *src, long long sp, int idx, bool ions, bool neutrals) {
     double um[NVM], uh[5], vm[NVM], vh[5];
     if (ions) {
@@ -734,19 +768,10 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
       for (int n = 0; n < 5; ++n) sV[(NVM + n) * RR + idx] = vh[n];
     }
   };
-  for (int u = tid; u < (SPLITP ? 2 : 1) * RR; u += NT) {
-    const int idx = SPLITP && u >= RR ? u - RR : u;
-    const bool ions = !SPLITP || u < RR, neutrals = !SPLITP || u >= RR;
-    const int ri = idx % RX - XO, rj = idx / RX;
-    if (XO && (ri < 0 || ri >= TX + 2 * kH)) continue;
-    // the corners only for the curl of B next to the tile's corner faces (resistivity)
-    if (NDIM == 2 && !RES && (ri < kH || ri >= TX + kH) && (rj < kH || rj >= TY + kH))
-      continue;
-    const int gi = i0 - kH + ri, gj = NDIM == 2 ? j0 - kH + rj : 0;
-    if (gi >= p.ix || gj >= p.jx) continue;
-    if (NDIM == 2 && staged) convert(sV + idx, RR, idx, ions, neutrals);
-    else convert(Us + (long long)gj * p.ix + gi, nc, idx, ions, neutrals);
-  }
+  tile_units([&](int idx, long long q, bool ions, bool neutrals) {
+    if (NDIM == 2 && (!RES || staged)) convert(sV + idx, RR, idx, ions, neutrals);
+    else convert(Us + q, nc, idx, ions, neutrals);
+  });
   };
   if (S == 0) {
     if (control) read_control();
@@ -767,7 +792,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     }
     // no copy in flight when the CTA leaves
     if (staged) tma_bar_wait(&s_bar, kTmaWaitLimit);
-    if (S == 1) cp_async_wait();
+    cp_async_wait();
     return;
   }
   const double dt = s_dt, cmax = s_cmax;
@@ -1574,18 +1599,26 @@ static cudaError_t set_stage_attr() {
   return cudaSuccess;
 }
 
-// Raises the dynamic shared-memory limit of every stage-kernel instance on the current
-// device; called once per context so that graph capture sees launches only.
-static cudaError_t prepare() {
+// Raises the dynamic shared-memory limit of the stage-kernel instances for p's dimension and
+// ion planes (p null: of every instance) on the current device; called once per context so
+// that graph capture sees launches only.  Setting the limit loads the instance, about 1 ms.
+static cudaError_t prepare(const KParams *p) {
   cudaError_t e;
 #if !PIP_HEAT_ONLY
-  if ((e = set_stage_attr<1, 8, 1>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr<1, 8, 2>()) != cudaSuccess) return e;
+  if (!p || p->ndim == 1) {
+    if ((e = set_stage_attr<1, 8, 1>()) != cudaSuccess) return e;
+    if ((e = set_stage_attr<1, 8, 2>()) != cudaSuccess) return e;
+  }
 #endif
-  if ((e = set_stage_attr<2, 8, 1>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr<2, 8, 2>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr<2, 9, 1>()) != cudaSuccess) return e;
-  return set_stage_attr<2, 9, 2>();
+  if (!p || (p->ndim == 2 && p->nvm == 8)) {
+    if ((e = set_stage_attr<2, 8, 1>()) != cudaSuccess) return e;
+    if ((e = set_stage_attr<2, 8, 2>()) != cudaSuccess) return e;
+  }
+  if (!p || (p->ndim == 2 && p->nvm == 9)) {
+    if ((e = set_stage_attr<2, 9, 1>()) != cudaSuccess) return e;
+    if ((e = set_stage_attr<2, 9, 2>()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // Whether a grid takes the small tiles (Tile<., 1>): while they all run at once.
