@@ -271,6 +271,9 @@ void build_kparams(pip_ctx *c) {
   k.nc = (long long)p.ix * p.jx;
   k.gm = p.gm;
   k.igm1 = 1.0 / (p.gm - 1.0);
+  k.gm_6 = p.gm / 6.0;
+  k.r3_gm = 3.0 / p.gm;
+  k.r_ro_lim = 1.0 / p.ro_lim;
   k.c32g = 3.0 / p.gm / 2.0;
   k.ro_lim = p.ro_lim;
   k.pr_lim = p.pr_lim;
@@ -357,6 +360,9 @@ int pip::kparams_from_params(const pip_params *p, KParams *k) {
   k->nc = (long long)p->ix * p->jx;
   k->gm = p->gm;
   k->igm1 = 1.0 / (p->gm - 1.0);
+  k->gm_6 = p->gm / 6.0;
+  k->r3_gm = 3.0 / p->gm;
+  k->r_ro_lim = 1.0 / p->ro_lim;
   k->c32g = 3.0 / p->gm / 2.0;
   k->ro_lim = p->ro_lim;
   k->pr_lim = p->pr_lim;

@@ -191,8 +191,7 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
         for (int n = 0; n < NVM; ++n) {
           const float *v = sV + n * RX + a;
           const float v0 = v[-1], v1 = v[0], v2 = v[1], v3 = v[2];
-          vl[n] = v1 + 0.5f * minmod<float>(v0, v1, v2);
-          vr[n] = v2 - 0.5f * minmod<float>(v1, v2, v3);
+          pair::face_states(v0, v1, v2, v3, vl[n], vr[n]);
         }
         vl[0] = fmaxf(vl[0], rolf);
         vr[0] = fmaxf(vr[0], rolf);
@@ -206,8 +205,7 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
         for (int n = 0; n < 5; ++n) {
           const float *v = sV + (NVM + n) * RX + a;
           const float v0 = v[-1], v1 = v[0], v2 = v[1], v3 = v[2];
-          vl[n] = v1 + 0.5f * minmod<float>(v0, v1, v2);
-          vr[n] = v2 - 0.5f * minmod<float>(v1, v2, v3);
+          pair::face_states(v0, v1, v2, v3, vl[n], vr[n]);
         }
         vl[0] = fmaxf(vl[0], rolf);
         vr[0] = fmaxf(vr[0], rolf);
@@ -248,9 +246,10 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
       if (p.ir) mixed::ir_rates<NVM>(a_m, p, gr, gion);
       if (p.imp && STAGE == 2) {
         double ds[5];
-        const Prim<double> qh = mixed::prim_hd(a_h, p);
-        const Prim<double> qm = mixed::prim_mhd<NVM>(a_m, p);
-        mixed::collision_ds<NVM>(a_m, a_h, qm, qh, p, dt_coll, ds);
+        double im, ih;
+        const Prim<double> qh = mixed::prim_hd(a_h, p, ih);
+        const Prim<double> qm = mixed::prim_mhd<NVM>(a_m, p, im);
+        mixed::collision_ds<NVM>(a_m, a_h, qm, qh, im, ih, p, dt_coll, ds);
 #pragma unroll
         for (int n = 0; n < 5; ++n) {
           a_h[n] = a_h[n] - dt_coll * ds[n];
@@ -259,10 +258,11 @@ __device__ void run_stage(const KParams &p, const float *Us, float *Ahi, float *
       }
       double S_m[5], S_h[5];
       {
-        const Prim<double> qh = mixed::prim_hd(s_h, p);
-        const Prim<double> qm = mixed::prim_mhd<NVM>(s_m, p);
+        double im, ih;
+        const Prim<double> qh = mixed::prim_hd(s_h, p, ih);
+        const Prim<double> qm = mixed::prim_mhd<NVM>(s_m, p, im);
         double ds[5];
-        mixed::collision_ds<NVM>(s_m, s_h, qm, qh, p, dt_coll, ds);
+        mixed::collision_ds<NVM>(s_m, s_h, qm, qh, im, ih, p, dt_coll, ds);
         if (p.imp) {
 #pragma unroll
           for (int n = 0; n < 5; ++n) {
@@ -361,8 +361,7 @@ __device__ void run_member_2d(const KParams &p, float *Ahi, float *Alo, float *B
   float *sV = smem;
   double *sD6 = reinterpret_cast<double *>(sV + NV2 * RR);
   double *sD9 = sD6 + (NVM2 == 9 ? NFX + NFY : 0);
-  float *sFx = reinterpret_cast<float *>(sD9 + (NVM2 == 9 ? NFX + NFY : 0));
-  float *sFy = sFx + NV2 * NFX;
+  float *sF = reinterpret_cast<float *>(sD9 + (NVM2 == 9 ? NFX + NFY : 0));
   const int tid = threadIdx.x;
   const long long nc = p.nc;
   const float gmf = (float)p.gm, rolf = (float)p.ro_lim, prlf = (float)p.pr_lim;
@@ -428,7 +427,7 @@ __device__ void run_member_2d(const KParams &p, float *Ahi, float *Alo, float *B
     for (int t = 0; t < ntiles; ++t) {
       const int i0 = p.m0 + (t % ntx) * TX2, j0 = p.m1 + (t / ntx) * TY2;
       mixed::tile_stage<2, NVM2, 1, TX2, TY2, NT, kH>(p, Ahi, Ahi, Alo, B, nullptr, i0, j0, dt, cmax,
-                                                     0, false, sV, sD6, sD9, sFx, sFy, d1, r1, g1,
+                                                     0, false, sV, sD6, sD9, sF, d1, r1, g1,
                                                      bad);
       __syncthreads();   // the next tile reuses the shared memory
     }
@@ -436,7 +435,7 @@ __device__ void run_member_2d(const KParams &p, float *Ahi, float *Alo, float *B
     for (int t = 0; t < ntiles; ++t) {
       const int i0 = p.m0 + (t % ntx) * TX2, j0 = p.m1 + (t / ntx) * TY2;
       mixed::tile_stage<2, NVM2, 2, TX2, TY2, NT, kH>(p, B, Ahi, Alo, Ahi, Alo, i0, j0, dt, cmax,
-                                                     last ? 1 : 2, false, sV, sD6, sD9, sFx, sFy,
+                                                     last ? 1 : 2, false, sV, sD6, sD9, sF,
                                                      d2, r2, g2, bad);
       __syncthreads();
     }

@@ -40,6 +40,8 @@ struct KParams {
   long long nc;      // ix*jx
   double gm, ro_lim, pr_lim, ac, safety;
   double igm1;       // 1/(gm-1)
+  double gm_6, r3_gm; // gm/6 and 3/gm (factors of the exponential exchange)
+  double r_ro_lim;    // 1/ro_lim
   double c32g;       // 3/gm/2 of the explicit collision energy term
   double sg_all;     // safety*min over all dx, dy, dz (numerator of cmax)
   double col_lim;    // min(safety,0.3) or pip_imp_factor (cfl_pn_col)

@@ -115,8 +115,7 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
   float *sV = reinterpret_cast<float *>(smd);
   double *sD6 = reinterpret_cast<double *>(sV + NV * RR);
   double *sD9 = sD6 + (NVM == 9 ? NFX + NFY : 0);
-  float *sFx = reinterpret_cast<float *>(sD9 + (NVM == 9 ? NFX + NFY : 0));
-  float *sFy = sFx + NV * NFX;
+  float *sF = reinterpret_cast<float *>(sD9 + (NVM == 9 ? NFX + NFY : 0));
   static_assert((NV * RR * sizeof(float)) % sizeof(double) == 0, "Dedner planes alignment");
   __shared__ __align__(8) unsigned long long s_bar;
   __shared__ double s_dt, s_cmax;
@@ -218,7 +217,7 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
   double dtc = 10.0, rhoc = 0.0, grc = 0.0;
   bool bad = false;
   tile_stage<NDIM, NVM, STAGE, TX, TY, NT, kH>(p, Us, U0hi, U0lo, Ohi, Olo, i0, j0, dt, s_cmax,
-                                              s_epi, staged, sV, sD6, sD9, sFx, sFy, dtc, rhoc,
+                                              s_epi, staged, sV, sD6, sD9, sF, dtc, rhoc,
                                               grc, bad);
   if (bad) atomicOr(&ctrl->nan_flag, 1);
   if (STAGE == 2 && s_epi == 2) block_reduce_cfl<NT>(dtc, rhoc, grc, ctrl, s_slot);

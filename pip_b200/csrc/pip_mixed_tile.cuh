@@ -28,11 +28,11 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
                                            const float *U0hi, const float *U0lo, float *Ohi,
                                            float *Olo, int i0, int j0, double dt, double cmax,
                                            int ep, bool staged, float *sV, double *sD6,
-                                           double *sD9, float *sFx, float *sFy, double &dtc,
+                                           double *sD9, float *sF, double &dtc,
                                            double &rhoc, double &grc, bool &bad) {
   constexpr int NV = NVM + 5;
   constexpr int RX = TX + 2 * kH, RY = NDIM == 2 ? TY + 2 * kH : 1, RR = RX * RY;
-  constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0;
+  constexpr int NFX = (TX + 1) * TY, NFY = NDIM == 2 ? TX * (TY + 1) : 0, NF = NFX + NFY;
   const int tid = threadIdx.x;
   const float gmf = (float)p.gm, rolf = (float)p.ro_lim, prlf = (float)p.pr_lim;
   const float igm1f = (float)p.igm1;
@@ -83,26 +83,19 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
   const int iend = p.m0 + p.nx, jend = NDIM == 2 ? p.m1 + p.ny : 1;
   for (int f = tid; f < NFX + NFY; f += NT) {
     // x faces first, then y faces, each in row order (constant divisors in each branch)
-    int a, s, py, fo, nf;
-    float *Fout;
+    int a, s, py;
     if (f < NFX) {
       const int fi = f % (TX + 1), fj = f / (TX + 1);
       if (i0 + fi - 1 >= iend || (NDIM == 2 && j0 + fj >= jend)) continue;
       a = (NDIM == 2 ? (fj + kH) * RX : 0) + fi + kH - 1;
       s = 1;
       py = 0;
-      Fout = sFx;
-      fo = f;
-      nf = NFX;
     } else {
       const int g = f - NFX, fi = g % TX, fj = g / TX;
       if (i0 + fi >= iend || j0 + fj - 1 >= jend) continue;
       a = (fj + kH - 1) * RX + fi + kH;
       s = RX;
       py = 1;
-      Fout = sFy;
-      fo = g;
-      nf = NFY;
     }
     {
       // the HLLD of planes 0-7; with Dedner cleaning the normal-field and psi fluxes are the
@@ -113,8 +106,7 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
         const int src = py ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
         const float *v = sV + src * RR + a;
         const float v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-        vl[n] = v1 + 0.5f * minmod<float>(v0, v1, v2);
-        vr[n] = v2 - 0.5f * minmod<float>(v1, v2, v3);
+        pair::face_states(v0, v1, v2, v3, vl[n], vr[n]);
       }
       vl[0] = fmaxf(vl[0], rolf);
       vr[0] = fmaxf(vr[0], rolf);
@@ -123,7 +115,7 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
       for (int n = 0; n < 8; ++n) {
         if (NVM == 9 && n == 5) continue;
         const int dst = py ? (n == 1 ? 2 : n == 2 ? 1 : n == 5 ? 6 : n == 6 ? 5 : n) : n;
-        Fout[dst * nf + fo] = fx[n];
+        sF[dst * NF + f] = fx[n];
       }
       if (NVM == 9) {
         // reconstruct Bn and psi in FP64 from the FP32 cell values
@@ -146,8 +138,7 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
         const int src = py ? (n == 1 ? 2 : n == 2 ? 1 : n) : n;
         const float *v = sV + (NVM + src) * RR + a;
         const float v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-        vl[n] = v1 + 0.5f * minmod<float>(v0, v1, v2);
-        vr[n] = v2 - 0.5f * minmod<float>(v1, v2, v3);
+        pair::face_states(v0, v1, v2, v3, vl[n], vr[n]);
       }
       vl[0] = fmaxf(vl[0], rolf);
       vr[0] = fmaxf(vr[0], rolf);
@@ -155,7 +146,7 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
 #pragma unroll
       for (int n = 0; n < 5; ++n) {
         const int dst = py ? (n == 1 ? 2 : n == 2 ? 1 : n) : n;
-        Fout[(NVM + dst) * nf + fo] = fx[n];
+        sF[(NVM + dst) * NF + f] = fx[n];
       }
     }
   }
@@ -195,9 +186,10 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
     if (p.ir) ir_rates<NVM>(a_m, p, gr, gion);
     if (p.imp && STAGE == 2) {
       double ds[5];
-      const Prim<double> qh = prim_hd(a_h, p);
-      const Prim<double> qm = prim_mhd<NVM>(a_m, p);
-      collision_ds<NVM>(a_m, a_h, qm, qh, p, dt_coll, ds);
+      double im, ih;
+      const Prim<double> qh = prim_hd(a_h, p, ih);
+      const Prim<double> qm = prim_mhd<NVM>(a_m, p, im);
+      collision_ds<NVM>(a_m, a_h, qm, qh, im, ih, p, dt_coll, ds);
 #pragma unroll
       for (int n = 0; n < 5; ++n) {
         a_h[n] = a_h[n] - dt_coll * ds[n];
@@ -206,10 +198,11 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
     }
     double S_m[5], S_h[5];
     {
-      const Prim<double> qh = prim_hd(s_h, p);
-      const Prim<double> qm = prim_mhd<NVM>(s_m, p);
+      double im, ih;
+      const Prim<double> qh = prim_hd(s_h, p, ih);
+      const Prim<double> qm = prim_mhd<NVM>(s_m, p, im);
       double ds[5];
-      collision_ds<NVM>(s_m, s_h, qm, qh, p, dt_coll, ds);
+      collision_ds<NVM>(s_m, s_h, qm, qh, im, ih, p, dt_coll, ds);
       if (p.imp) {
 #pragma unroll
         for (int n = 0; n < 5; ++n) {
@@ -246,10 +239,10 @@ __device__ __forceinline__ void tile_stage(const KParams &p, const float *__rest
       const bool dy64 = NVM == 9 && (n == 6 || n == NVM - 1);
       const double *Dx = n == NVM - 1 ? sD9 : sD6;
       if (dx64) u -= cx * (Dx[fxl + 1] - Dx[fxl]);
-      else u -= cx * (double)(sFx[n * NFX + fxl + 1] - sFx[n * NFX + fxl]);
+      else u -= cx * (double)(sF[n * NF + fxl + 1] - sF[n * NF + fxl]);
       if (NDIM == 2) {
         if (dy64) u -= cy * (Dx[NFX + fyl + TX] - Dx[NFX + fyl]);
-        else u -= cy * (double)(sFy[n * NFY + fyl + TX] - sFy[n * NFY + fyl]);
+        else u -= cy * (double)(sF[n * NF + NFX + fyl + TX] - sF[n * NF + NFX + fyl]);
       }
       if (n < NVM) {
         if (n < 5) u += S_m[n] * dt_sub;

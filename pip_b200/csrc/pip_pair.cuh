@@ -34,6 +34,15 @@ PIP_HD float2 fma2(float2 a, float2 b, float2 c) {
 // a - b, rounded once (b * -1 is exact)
 PIP_HD float2 sub2(float2 a, float2 b) { return fma2(b, s2(-1.0f), a); }
 
+// Face states between cells 1 and 2 of four cells in a row: v1 + minmod/2, v2 - minmod/2 as
+// minmod<float> forms them.  The limited slope is symmetric in its two differences, so the sign
+// and the magnitude of the difference across the face serve both sides.
+PIP_HD void face_states(float v0, float v1, float v2, float v3, float &l, float &r) {
+  const float b = v2 - v1, sg = rsign1(b), h = 0.5f * sg, m = rabs(b);
+  l = v1 + h * rmax(0.0f, rmin(m, sg * (v1 - v0)));
+  r = v2 - h * rmax(0.0f, rmin(m, sg * (v3 - v2)));
+}
+
 // hllc_flux_rcp<float> (HLL_rot.f90:615-687) with paired left/right work.
 PIP_HD void hllc_flux(const float (&v_l)[5], const float (&v_r)[5],
                                           float (&flx)[5], float gm, float igm1) {
