@@ -1,7 +1,7 @@
 // pip_fp64_forms.cuh -- device forms of the FP64 solvers for the FMA-contracted build.
 //
 // The stage kernels of that build are bound by the instructions they issue (FP64 pipe 45 %,
-// issue 55 % busy at 16 warps per SM), so these forms reach the results of the literal ones
+// issue 57 % busy at 16 warps per SM, DRAM 15-22 %), so these forms reach the results of the literal ones
 // (pip_physics.cuh) with fewer operations:
 //   * minmod by selection instead of min/max/sign products (the same value bit for bit);
 //   * HLLC and HLLD evaluate one side of the contact only (the one the face flux is taken
@@ -14,10 +14,11 @@
 // Every sum that must cancel to +0 at a mirror wall is made of separately rounded products
 // (mul_rn, see pip_physics.cuh).  Against the literal forms a flux differs by rounding.
 //
-// Measured on a B200, per step of two stage launches, before -> after: Orszag-Tang 1024^2
-// 0.551 -> 0.370 ms; 517x333 with walls and the exponential collisions 124 -> 85 us; 1024
-// cells in 1D 27.3 -> 20.5 us (a chain of dependent operations there).  Error of the state
-// against 64-bit torch after 100 steps: 3.8e-15 -> 3.2e-15.
+// Measured on a B200, per step of two stage launches, the literal forms -> these, nothing else
+// changed: Orszag-Tang 1024^2 0.551 -> 0.370 ms; 517x333 with walls and the exponential
+// collisions 124 -> 85 us; 1024 cells in 1D 27.3 -> 20.5 us (a chain of dependent operations
+// there).  With the other changes of the stage kernels 0.310 ms, 67 us and 8.2 us.  Error of the
+// state against 64-bit torch after 100 steps: 3.8e-15 -> 3.2e-15.
 #pragma once
 
 #include "pip_kernels.cuh"
@@ -28,8 +29,8 @@ namespace pip {
 // Below this the roots' argument is taken as zero (their seed flushes subnormals).
 constexpr double kTinyRoot = 1.0e-280;
 
-// 1/sqrt(x) for x >= 0 (x below kTinyRoot as kTinyRoot, so that 0 * rsqrt_nr(0) is 0): the hardware's approximate inverse square root (PTX
-// rsqrt.approx.ftz.f64) and two Newton-Raphson steps y <- y + y (1/2 - x/2 y^2).
+// 1/sqrt(x) for x >= 0 (x below kTinyRoot as kTinyRoot, so that 0 * rsqrt_nr(0) is 0): the
+// hardware's approximate inverse square root (PTX rsqrt.approx.ftz.f64) and two Newton-Raphson steps y <- y + y (1/2 - x/2 y^2).
 __device__ __forceinline__ double rsqrt_nr(double x) {
   x = x > kTinyRoot ? x : kTinyRoot;
   double y;

@@ -6,7 +6,7 @@
 // shear layer stop after other iteration counts, the temperatures differ by 1e-10, and the
 // HLLD states' jumps carry single cells of the field to 6e-8 within ten steps.  These
 // kernels keep the trajectories of conduction runs bit for bit; the stages are a quarter of
-// such a step (1.1 of 4.1 ms), so the faster forms would give it 6 %.
+// such a step (about 1 of 3.9 ms), so the faster forms would give it 6 %.
 #define PIP_FLAVOUR heat
 #define PIP_RCP 1
 #define PIP_FAST 0
