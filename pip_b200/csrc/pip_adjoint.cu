@@ -59,6 +59,28 @@ struct CandPart {
   int rsp;    // species of rmax: 0 ions, 1 neutrals
 };
 
+// The reverse sweep's kernels are programmatic dependents of one another: a kernel's blocks start
+// while the previous one's last blocks run, and touch no memory before this wait, which returns
+// when every earlier kernel of the stream is done.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 __device__ __forceinline__ bool interior(const KParams &p, int i, int j) {
   return i >= p.m0 && i < p.m0 + p.nx && (p.ndim == 1 || (j >= p.m1 && j < p.m1 + p.ny));
 }
@@ -193,6 +215,7 @@ __device__ __forceinline__ void gather_dir(const double *__restrict__ gL, const 
 
 // Primitives of every cell (u2v_mhd / u2v_hd, HLL_rot.f90:1136-1186).
 __global__ void u2v_kernel(const KParams p, const double *__restrict__ U, double *__restrict__ V) {
+  pdl_begin();
   const long long nc = p.nc;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nc;
        q += (long long)gridDim.x * blockDim.x) {
@@ -227,6 +250,7 @@ face_vjp_kernel(const KParams p, const double *__restrict__ V, const double *__r
                 unsigned long long *my, double *part_dot, double *part_dac) {
   constexpr int N0 = SP == 0 ? 0 : NVM, N1 = SP == 0 ? NVM : NV;
   __shared__ double s_red[NT / 32];
+  pdl_begin();
   const long long nc = p.nc;
   const double dt_sub = fac * (*dtp);
   const long long nfx = (long long)p.jx * (p.ix - 1);
@@ -312,6 +336,7 @@ cell_vjp_kernel(const KParams p, const double *__restrict__ Us, const double *__
   __shared__ double s_red[4][NT / 32];
   __shared__ long long s_idx[2][NT / 32];
   __shared__ int s_kind[2][NT / 32];
+  pdl_begin();
   const int tid = threadIdx.x;
   const double dt_sub = fac * (*dtp);
   const long long nc = p.nc;
@@ -467,6 +492,7 @@ cell_vjp_kernel(const KParams p, const double *__restrict__ Us, const double *__
 __global__ void __launch_bounds__(256) fold_kernel(double *lam, long long nc, const int *cells,
                                                    const int *src, const unsigned short *neg,
                                                    int ncells, int nent) {
+  pdl_begin();
   const long long total = (long long)ncells * NV;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -493,6 +519,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(const KParams p, int nb, 
   __shared__ double s_a[256], s_b[256], s_c[256], s_r[256];
   __shared__ long long s_ci[256], s_ri[256];
   __shared__ int s_ck[256], s_rs[256];
+  pdl_begin();
   const int t = threadIdx.x;
   double sd = 0.0, sa = 0.0, cm = 1.0e300, rm = -1.0e300;
   long long ci = -1, ri = -1;
@@ -587,16 +614,20 @@ cudaError_t launch_stage_vjp(const KParams &p, const double *Us, const double *l
                              double *pdot, double *pdac, int nbf, CandPart *cand, cudaStream_t s) {
   const long long nc = p.nc;
   const int gu = (int)std::min<long long>((nc + 255) / 256, 148 * 8);
-  u2v_kernel<<<gu, 256, 0, s>>>(p, Us, V);
-  face_vjp_kernel<0, kFaceThreads><<<nbf, kFaceThreads, 0, s>>>(p, V, lam, dtp, fac, gx, mx, gy,
-                                                                my, pdot, pdac);
+  cudaError_t e;
+  if ((e = launch_pdl(u2v_kernel, gu, 256, s, p, Us, V)) != cudaSuccess) return e;
+  if ((e = launch_pdl(face_vjp_kernel<0, kFaceThreads>, nbf, kFaceThreads, s, p, (const double *)V,
+                      lam, dtp, fac, gx, mx, gy, my, pdot, pdac)) != cudaSuccess)
+    return e;
   const int nbh = face_blocks_h(p);
-  face_vjp_kernel<1, kFaceThreadsH><<<nbh, kFaceThreadsH, 0, s>>>(p, V, lam, dtp, fac, gx, mx, gy,
-                                                                  my, pdot + nbf, pdac + nbf);
+  if ((e = launch_pdl(face_vjp_kernel<1, kFaceThreadsH>, nbh, kFaceThreadsH, s, p,
+                      (const double *)V, lam, dtp, fac, gx, mx, gy, my, pdot + nbf, pdac + nbf)) !=
+      cudaSuccess)
+    return e;
   const int nbc = (int)((nc + kCellThreads - 1) / kCellThreads);
-  cell_vjp_kernel<<<nbc, kCellThreads, 0, s>>>(p, Us, lam, acc, out, dtp, fac, gx, mx, gy, my,
-                                               pdot + nbf + nbh, pdac + nbf + nbh, cand);
-  return cudaGetLastError();
+  return launch_pdl(cell_vjp_kernel, nbc, kCellThreads, s, p, Us, lam, acc, out, dtp, fac,
+                    (const double *)gx, (const unsigned long long *)mx, (const double *)gy,
+                    (const unsigned long long *)my, pdot + nbf + nbh, pdac + nbf + nbh, cand);
 }
 
 long long face_count(const KParams &p) {
@@ -738,8 +769,9 @@ FoldPlan fold_plan(const KParams &k) {
 
 void fold(pip_adj *a, double *lam, int grid) {
   if (a->nfold > 0)
-    pip::adjk::fold_kernel<<<grid, 256, 0, a->stream>>>(lam, a->kp.nc, a->d_fold, a->d_fsrc,
-                                                       a->d_fneg, a->nfold, a->nfent);
+    pip::adjk::launch_pdl(pip::adjk::fold_kernel, grid, 256, a->stream, lam, a->kp.nc,
+                          (const int *)a->d_fold, (const int *)a->d_fsrc,
+                          (const unsigned short *)a->d_fneg, a->nfold, a->nfent);
 }
 
 cudaError_t launch_vjp(pip_adj *a, int stage, const double *Us, const double *lam, const double *acc,
@@ -1028,10 +1060,11 @@ int pip_adj_backward(pip_adj *a, const double *gN, double *g0, double *g_col, fl
       fold(a, a->Lb, gf);
       ACK(cudaGetLastError());
       ACK(launch_vjp(a, 1, zp(s, j), a->Lb, a->La, a->La, dtp));
-      pip::adjk::finalize_kernel<<<1, 256, 0, a->stream>>>(kp, a->nb, a->nbc, a->p1dot, a->p1dac, a->p2dot,
-                                                            a->p2dac, a->cand, dtp, zp(s, j), a->La,
-                                                            a->dcol, nullptr);
-      ACK(cudaGetLastError());
+      ACK(pip::adjk::launch_pdl(pip::adjk::finalize_kernel, 1, 256, a->stream, kp, a->nb, a->nbc,
+                                (const double *)a->p1dot, (const double *)a->p1dac,
+                                (const double *)a->p2dot, (const double *)a->p2dac,
+                                (const CandPart *)a->cand, dtp, (const double *)zp(s, j), a->La,
+                                a->dcol, (double *)nullptr));
     }
     ACK(cudaEventRecord(a->ev_rev[s % 2], a->stream));
   }
