@@ -213,6 +213,13 @@ __device__ __forceinline__ void gather_dir(const double *__restrict__ gL, const 
   }
 }
 
+// A step's dt between the control block and the history: a kernel, because a copy between the
+// stages would end the chain of programmatic launches.
+__global__ void copy_dt_kernel(const double *src, double *dst) {
+  pdl_begin();
+  *dst = *src;
+}
+
 // Primitives of every cell (u2v_mhd / u2v_hd, HLL_rot.f90:1136-1186).
 __global__ void u2v_kernel(const KParams p, const double *__restrict__ U, double *__restrict__ V) {
   pdl_begin();
@@ -980,8 +987,8 @@ int pip_adj_forward(pip_adj *a, const double *U0, double *UN, int64_t nsteps, fl
     if (n % a->K == 0)
       ACK(cudaMemcpyAsync(a->ckpt[n / a->K], a->A, sb, cudaMemcpyDeviceToDevice, a->stream));
     ACK(a->L->stage(a->kp, 1, a->A, a->A, a->B, a->ctrl, 1, 0, a->stream, nullptr, 0));
-    ACK(cudaMemcpyAsync(a->dt_hist + n, &a->ctrl->dt, sizeof(double), cudaMemcpyDeviceToDevice,
-                        a->stream));
+    ACK(pip::adjk::launch_pdl(pip::adjk::copy_dt_kernel, 1, 1, a->stream,
+                              (const double *)&a->ctrl->dt, a->dt_hist + n));
     ACK(a->L->stage(a->kp, 2, a->B, a->A, a->A, a->ctrl, 1, -1, a->stream, nullptr, 0));
   }
   ACK(cudaMemcpyAsync(UN, a->A, sb, cudaMemcpyDeviceToDevice, a->stream));
@@ -1033,8 +1040,8 @@ int pip_adj_backward(pip_adj *a, const double *gN, double *g0, double *g_col, fl
     if (s + 2 < nseg) ACK(cudaStreamWaitEvent(a->stream2, a->ev_rev[s % 2], 0));
     // z_n, U1_n of the segment with the recorded dt
     for (int j = 0; j < len; ++j) {
-      ACK(cudaMemcpyAsync(&a->ctrl->dt, a->dt_hist + n0 + j, sizeof(double), cudaMemcpyDeviceToDevice,
-                          a->stream2));
+      ACK(pip::adjk::launch_pdl(pip::adjk::copy_dt_kernel, 1, 1, a->stream2,
+                                (const double *)(a->dt_hist + n0 + j), &a->ctrl->dt));
       ACK(a->L->stage(kp, 1, zp(s, j), zp(s, j), a->segu[s % 2][j], a->ctrl, 0, 0, a->stream2, nullptr, 0));
       if (j + 1 < len)
         ACK(a->L->stage(kp, 2, a->segu[s % 2][j], zp(s, j), zp(s, j + 1), a->ctrl, 0, 2, a->stream2, nullptr, 0));
