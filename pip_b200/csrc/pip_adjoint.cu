@@ -91,14 +91,6 @@ __device__ __forceinline__ int perm_m(int n) {
 }
 __device__ __forceinline__ int perm_h(int n) { return n == 1 ? 2 : n == 2 ? 1 : n; }
 
-// minmod(v0, v1, v2)'s slope and the branch taken (adj::minmod_mode's, by selection)
-__device__ __forceinline__ double minmod_branch(double v0, double v1, double v2, int &mode) {
-  const double X = v2 - v1, Y = v1 - v0;
-  const bool x = fabs(X) <= fabs(Y), on = X * Y > 0.0;
-  mode = on ? (x ? 1 : 2) : 0;
-  return on ? (x ? X : Y) : 0.0;
-}
-
 // minmod derivative of the slope at cell 1 of (v0, v1, v2) with respect to v_q
 __device__ __forceinline__ double dmm(int mode, int q) {
   if (mode == 1) return q == 1 ? -1.0 : (q == 2 ? 1.0 : 0.0);
@@ -127,10 +119,10 @@ __device__ __forceinline__ double face_vjp(const KParams &p, const double *__res
       const int src = ydir ? perm_m(n) : n;
       const double *v = V + src * RR + a;
       const double v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-      int mL, mR;
-      vl[n] = v1 + 0.5 * minmod_branch(v0, v1, v2, mL);
-      vr[n] = v2 - 0.5 * minmod_branch(v1, v2, v3, mR);
+      const int mL = adj::minmod_mode(v0, v1, v2), mR = adj::minmod_mode(v1, v2, v3);
       modes |= (unsigned long long)(mL | (mR << 2)) << (4 * src);
+      vl[n] = v1 + 0.5 * minmod<double>(v0, v1, v2);
+      vr[n] = v2 - 0.5 * minmod<double>(v1, v2, v3);
       af[n] = lamF[src];
       avl[n] = 0.0;
       avr[n] = 0.0;
@@ -155,10 +147,10 @@ __device__ __forceinline__ double face_vjp(const KParams &p, const double *__res
       const int src = ydir ? perm_h(n) : n;
       const double *v = V + (NVM + src) * RR + a;
       const double v0 = v[-s], v1 = v[0], v2 = v[s], v3 = v[2 * s];
-      int mL, mR;
-      vl[n] = v1 + 0.5 * minmod_branch(v0, v1, v2, mL);
-      vr[n] = v2 - 0.5 * minmod_branch(v1, v2, v3, mR);
+      const int mL = adj::minmod_mode(v0, v1, v2), mR = adj::minmod_mode(v1, v2, v3);
       modes |= (unsigned long long)(mL | (mR << 2)) << (4 * (NVM + src));
+      vl[n] = v1 + 0.5 * minmod<double>(v0, v1, v2);
+      vr[n] = v2 - 0.5 * minmod<double>(v1, v2, v3);
       af[n] = lamF[NVM + src];
       avl[n] = 0.0;
       avr[n] = 0.0;
@@ -231,8 +223,8 @@ __global__ void u2v_kernel(const KParams p, const double *__restrict__ U, double
     for (int n = 0; n < 8; ++n) um[n] = U[q + n * nc];
 #pragma unroll
     for (int n = 0; n < 5; ++n) uh[n] = U[q + (NVM + n) * nc];
-    u2v_mhd_fast<8>(um, vm, p.gm, p.ro_lim, p.pr_lim);
-    u2v_hd_fast(uh, vh, p.gm, p.ro_lim, p.pr_lim);
+    u2v_mhd<double, 8>(um, vm, p.gm, p.ro_lim, p.pr_lim);
+    u2v_hd<double>(uh, vh, p.gm, p.ro_lim, p.pr_lim);
 #pragma unroll
     for (int n = 0; n < 8; ++n) V[q + n * nc] = vm[n];
 #pragma unroll
@@ -293,11 +285,11 @@ face_vjp_kernel(const KParams p, const double *__restrict__ V, const double *__r
     } else {
       double ca = 0.0, cb = 0.0;
       if (!ydir) {
-        if (in_a) ca = dt_sub * rcp_(p.dx[ia]);
-        if (in_b) cb = dt_sub * rcp_(p.dx[ib]);
+        if (in_a) ca = dt_sub / p.dx[ia];
+        if (in_b) cb = dt_sub / p.dx[ib];
       } else {
-        if (in_a) ca = dt_sub * rcp_(p.dy[ja]);
-        if (in_b) cb = dt_sub * rcp_(p.dy[jb]);
+        if (in_a) ca = dt_sub / p.dy[ja];
+        if (in_b) cb = dt_sub / p.dy[jb];
       }
       double lamF[NV];
 #pragma unroll

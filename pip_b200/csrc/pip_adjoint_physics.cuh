@@ -11,31 +11,9 @@
 #pragma once
 
 #include "pip_physics.cuh"
-#if defined(__CUDACC__)
-#include "pip_fp64_forms.cuh"
-#endif
 
 namespace pip {
 namespace adj {
-
-// Quotients are products with rcp_, roots Newton's (pip_fp64_forms.cuh) on the device; the
-// host's are IEEE.  The face kernel of the ions is bound by its registers (255, 2 CTAs of 128
-// threads per SM) and by dependent FP64 latency; inline refined seeds instead of the
-// division and root routines took it from 55.0 to 45.9 us at 512x256.
-PIP_HD double root_(double x) {
-#if defined(__CUDA_ARCH__)
-  return sqrt_nr(x);
-#else
-  return std::sqrt(x);
-#endif
-}
-PIP_HD double rroot_(double x) {
-#if defined(__CUDA_ARCH__)
-  return rsqrt_nr(x);
-#else
-  return 1.0 / std::sqrt(x);
-#endif
-}
 
 // derivative of |x| (0 at x == 0)
 PIP_HD double dabs(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); }
@@ -46,7 +24,7 @@ PIP_HD double dabs(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); }
 PIP_HD void u2v_mhd_vjp(const double (&u)[8], const double (&a_v)[8], double gm, double ro_lim,
                         double pr_lim, double (&a_u)[8]) {
   const double ro = rmax(u[0], ro_lim);
-  const double roi = rcp_(ro);
+  const double roi = 1.0 / ro;
   const double m2 = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
   const double pr = (gm - 1.0) * (u[4] - 0.5 * m2 * roi - 0.5 * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]));
   const double a_pr = pr < pr_lim ? 0.0 : a_v[4];
@@ -65,7 +43,7 @@ PIP_HD void u2v_mhd_vjp(const double (&u)[8], const double (&a_v)[8], double gm,
 PIP_HD void u2v_hd_vjp(const double (&u)[5], const double (&a_v)[5], double gm, double ro_lim,
                        double pr_lim, double (&a_u)[5]) {
   const double ro = rmax(u[0], ro_lim);
-  const double roi = rcp_(ro);
+  const double roi = 1.0 / ro;
   const double m2 = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
   const double pr = (gm - 1.0) * (u[4] - 0.5 * m2 * roi);
   const double a_pr = pr < pr_lim ? 0.0 : a_v[4];
@@ -86,7 +64,7 @@ template <int N, int NB>
 PIP_HD void cq2pv_vjp(const double (&u)[N], const double (&a_w)[5], const double (&a_q)[5],
                       double gm, double igm1, double ro_lim, double pr_lim, double (&a_u)[N]) {
   const double de = u[0];
-  const double inv = rcp_(de);
+  const double inv = 1.0 / de;
   double v[3] = {u[1] * inv, u[2] * inv, u[3] * inv};
   const double kin = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   double bb = 0.0;
@@ -168,8 +146,8 @@ PIP_HD void hllc_vjp(const double (&vl)[5], const double (&vr)[5], const double 
   fl[2] = ul[2] * vnl; fr[2] = ur[2] * vnr;
   fl[3] = ul[3] * vnl; fr[3] = ur[3] * vnr;
   fl[4] = (ul[4] + prl) * vnl; fr[4] = (ur[4] + prr) * vnr;
-  const double Xl = gm * prl * rcp_(vl[0]), Xr = gm * prr * rcp_(vr[0]);
-  const double csl = root_(Xl), csr = root_(Xr);
+  const double Xl = gm * prl / vl[0], Xr = gm * prr / vr[0];
+  const double csl = rsqrt_(Xl), csr = rsqrt_(Xr);
   const bool sl_left = (vnl - csl) <= (vnr - csr);
   const bool sr_left = (vnl + csl) >= (vnr + csr);
   const double sl = kHllcAcc * (sl_left ? vnl - csl : vnr - csr);
@@ -177,9 +155,9 @@ PIP_HD void hllc_vjp(const double (&vl)[5], const double (&vr)[5], const double 
   const double ql = ul[0] * (sl - vnl), qr = ur[0] * (sr - vnr);
   const double Nn = mul_rn(ur[1], sr - vnr) - mul_rn(ul[1], sl - vnl) + prl - prr;
   const double Dd = qr - ql;
-  const double sm = Nn * rcp_(Dd);
+  const double sm = Nn / Dd;
   const double prm = sm * ql - ul[1] * (sl - vnl) + prl;
-  const double il = rcp_(sl - sm), ir = rcp_(sr - sm);
+  const double il = 1.0 / (sl - sm), ir = 1.0 / (sr - sm);
   stl[0] = ql * il; str[0] = qr * ir;
   stl[1] = stl[0] * sm; str[1] = str[0] * sm;
   stl[2] = stl[0] * vl[2]; str[2] = str[0] * vr[2];
@@ -261,8 +239,8 @@ PIP_HD void hllc_vjp(const double (&vl)[5], const double (&vr)[5], const double 
   a_vnl += ul[1] * a_prm;
   a_prl += a_prm;
   // sm = Nn / Dd
-  const double a_N = a_sm * rcp_(Dd);
-  const double a_D = -sm * rcp_(Dd) * a_sm;
+  const double a_N = a_sm / Dd;
+  const double a_D = -sm / Dd * a_sm;
   a_qr += a_D;
   a_ql -= a_D;
   a_ur[1] += (sr - vnr) * a_N;
@@ -287,14 +265,14 @@ PIP_HD void hllc_vjp(const double (&vl)[5], const double (&vr)[5], const double 
   if (sr_left) { a_vnl += kHllcAcc * a_sr; a_csl += kHllcAcc * a_sr; }
   else { a_vnr += kHllcAcc * a_sr; a_csr += kHllcAcc * a_sr; }
   if (csl > 0.0) {
-    const double aX = a_csl * rcp_(2.0 * csl);
-    a_prl += gm * rcp_(vl[0]) * aX;
-    a_vl[0] -= Xl * rcp_(vl[0]) * aX;
+    const double aX = a_csl / (2.0 * csl);
+    a_prl += gm / vl[0] * aX;
+    a_vl[0] -= Xl / vl[0] * aX;
   }
   if (csr > 0.0) {
-    const double aX = a_csr * rcp_(2.0 * csr);
-    a_prr += gm * rcp_(vr[0]) * aX;
-    a_vr[0] -= Xr * rcp_(vr[0]) * aX;
+    const double aX = a_csr / (2.0 * csr);
+    a_prr += gm / vr[0] * aX;
+    a_vr[0] -= Xr / vr[0] * aX;
   }
   // physical fluxes
   a_ul[1] += a_fl[0] + vnl * a_fl[1];
@@ -339,7 +317,7 @@ PIP_HD void star_forward(const double (&v)[8], const double (&u)[8], double S, d
   st.iS = iS;
   st.d = v[0] * (S - v[1]);
   st.den = st.d * (S - sm) - bn2;
-  st.f1 = rcp_(st.den);
+  st.f1 = 1.0 / st.den;
   st.num = st.d * (S - v[1]) - bn2;
   st.g = st.f1 * st.num;
   st.u1[5] = bn;
@@ -458,14 +436,14 @@ PIP_HD int hlld_vjp(const double (&vl)[8], const double (&vr)[8], const double (
   fr[7] = vr[1] * vr[7] - vr[5] * vr[3];
   const double f1l = gm * vl[4], Al = f1l + b2l;
   const double discl = Al * Al - 4.0 * f1l * (vl[5] * vl[5]);
-  const double ddl = root_(rmax(discl, 0.0));
-  const double Ql = (Al + ddl) * rcp_(2.0 * vl[0]);
-  const double vfl = root_(Ql);
+  const double ddl = rsqrt_(rmax(discl, 0.0));
+  const double Ql = (Al + ddl) / (2.0 * vl[0]);
+  const double vfl = rsqrt_(Ql);
   const double f1r = gm * vr[4], Ar = f1r + b2r;
   const double discr = Ar * Ar - 4.0 * f1r * (vr[5] * vr[5]);
-  const double ddr = root_(rmax(discr, 0.0));
-  const double Qr = (Ar + ddr) * rcp_(2.0 * vr[0]);
-  const double vfr = root_(Qr);
+  const double ddr = rsqrt_(rmax(discr, 0.0));
+  const double Qr = (Ar + ddr) / (2.0 * vr[0]);
+  const double vfr = rsqrt_(Qr);
   const bool vmin_left = vl[1] <= vr[1];
   const bool vmax_left = vl[1] >= vr[1];
   const bool vf_left = vfl >= vfr;
@@ -490,19 +468,19 @@ PIP_HD int hlld_vjp(const double (&vl)[8], const double (&vr)[8], const double (
       if (flx_out) flx_out[n] = fr[n];
     }
   } else {
-    const double f1 = rcp_(sr - sl);
+    const double f1 = 1.0 / (sr - sl);
     double uh[8], w[8];
     for (int n = 0; n < 8; ++n) {
       w[n] = mul_rn(sr, ur[n]) - mul_rn(sl, ul[n]) - fr[n] + fl[n];
       uh[n] = f1 * w[n];
     }
-    const double iuh0 = rcp_(uh[0]);
+    const double iuh0 = 1.0 / uh[0];
     const double sm = uh[1] * iuh0;
     const double pt = ptl + vl[0] * (sl - vl[1]) * (sm - vl[1]);
-    const double ilm = rcp_(sl - sm), irm = rcp_(sr - sm);
+    const double ilm = 1.0 / (sl - sm), irm = 1.0 / (sr - sm);
     const double rol1 = vl[0] * (sl - vl[1]) * ilm;
     const double ror1 = vr[0] * (sr - vr[1]) * irm;
-    const double rsl = rroot_(rol1), rsr = rroot_(ror1);
+    const double rsl = rrsqrt(rol1), rsr = rrsqrt(ror1);
     const double bn = uh[5], bn2 = bn * bn;
     const double sal = rabs(bn) * rsl, sar = rabs(bn) * rsr;
 
@@ -612,7 +590,7 @@ PIP_HD int hlld_vjp(const double (&vl)[8], const double (&vr)[8], const double (
         // central states (HLL_rot.f90:861-898)
         const double rols = rol1 * rsl, rors = ror1 * rsr;
         const double s = rols + rors;
-        const double f1c = rcp_(s);
+        const double f1c = 1.0 / s;
         const double f2 = rsign1(bn);
         const double Y = rols * L.vy1 + rors * Rt.vy1 + (Rt.u1[6] - L.u1[6]) * f2;
         const double Z = rols * L.vz1 + rors * Rt.vz1 + (Rt.u1[7] - L.u1[7]) * f2;
@@ -792,12 +770,12 @@ PIP_HD int hlld_vjp(const double (&vl)[8], const double (&vr)[8], const double (
     const double a_vfl = vf_left ? a_vfm : 0.0, a_vfr = vf_left ? 0.0 : a_vfm;
     double a_b2l = 0.0, a_b2r = 0.0;
     if (vfl > 0.0 && a_vfl != 0.0) {
-      const double aQ = a_vfl * rcp_(2.0 * vfl);
-      double a_A = aQ * rcp_(2.0 * vl[0]);
-      const double a_dd = aQ * rcp_(2.0 * vl[0]);
-      a_vl[0] -= Ql * rcp_(vl[0]) * aQ;
+      const double aQ = a_vfl / (2.0 * vfl);
+      double a_A = aQ / (2.0 * vl[0]);
+      const double a_dd = aQ / (2.0 * vl[0]);
+      a_vl[0] -= Ql / vl[0] * aQ;
       if (discl > 0.0) {
-        const double a_disc = a_dd * rcp_(2.0 * ddl);
+        const double a_disc = a_dd / (2.0 * ddl);
         a_A += 2.0 * Al * a_disc;
         const double a_f1 = -4.0 * (vl[5] * vl[5]) * a_disc;
         a_vl[5] += -8.0 * f1l * vl[5] * a_disc;
@@ -808,12 +786,12 @@ PIP_HD int hlld_vjp(const double (&vl)[8], const double (&vr)[8], const double (
       a_b2l += a_A;
     }
     if (vfr > 0.0 && a_vfr != 0.0) {
-      const double aQ = a_vfr * rcp_(2.0 * vfr);
-      double a_A = aQ * rcp_(2.0 * vr[0]);
-      const double a_dd = aQ * rcp_(2.0 * vr[0]);
-      a_vr[0] -= Qr * rcp_(vr[0]) * aQ;
+      const double aQ = a_vfr / (2.0 * vfr);
+      double a_A = aQ / (2.0 * vr[0]);
+      const double a_dd = aQ / (2.0 * vr[0]);
+      a_vr[0] -= Qr / vr[0] * aQ;
       if (discr > 0.0) {
-        const double a_disc = a_dd * rcp_(2.0 * ddr);
+        const double a_disc = a_dd / (2.0 * ddr);
         a_A += 2.0 * Ar * a_disc;
         const double a_f1 = -4.0 * (vr[5] * vr[5]) * a_disc;
         a_vr[5] += -8.0 * f1r * vr[5] * a_disc;
@@ -893,8 +871,8 @@ PIP_HD double collision_vjp(const double (&um)[8], const double (&uh)[5], const 
   for (int n = 0; n < 5; ++n) wh[n] = uh[n];
   const Prim<double> qm = cq2pv_mhd_rcp<double, 8>(wm, gm, igm1, ro_lim, pr_lim);
   const Prim<double> qh = cq2pv_hd_rcp<double>(wh, gm, igm1, ro_lim, pr_lim);
-  const double te = qm.pr * rcp_(qm.de) * gm * kMuP;
-  const double nte = qh.pr * rcp_(qh.de) * gm * kMuN;
+  const double te = qm.pr / qm.de * gm * kMuP;
+  const double nte = qh.pr / qh.de * gm * kMuN;
   const double c32g = 3.0 / gm / 2.0;
   const double Qb = 0.5 * ((qh.vx * qh.vx - qm.vx * qm.vx) + (qh.vy * qh.vy - qm.vy * qm.vy) +
                            (qh.vz * qh.vz - qm.vz * qm.vz)) +
@@ -919,10 +897,10 @@ PIP_HD double collision_vjp(const double (&um)[8], const double (&uh)[5], const 
     a_qh[1] += qh.vx * aQ; a_qh[2] += qh.vy * aQ; a_qh[3] += qh.vz * aQ;
     a_qm[1] -= qm.vx * aQ; a_qm[2] -= qm.vy * aQ; a_qm[3] -= qm.vz * aQ;
     const double a_nte = c32g * aQ, a_te = -c32g * aQ;
-    a_qm[4] += gm * kMuP * rcp_(qm.de) * a_te;
-    a_qm[0] -= te * rcp_(qm.de) * a_te;
-    a_qh[4] += gm * kMuN * rcp_(qh.de) * a_nte;
-    a_qh[0] -= nte * rcp_(qh.de) * a_nte;
+    a_qm[4] += gm * kMuP / qm.de * a_te;
+    a_qm[0] -= te / qm.de * a_te;
+    a_qh[4] += gm * kMuN / qh.de * a_nte;
+    a_qh[0] -= nte / qh.de * a_nte;
   }
   cq2pv_vjp<8, 3>(um, a_wm, a_qm, gm, igm1, ro_lim, pr_lim, a_um);
   cq2pv_vjp<5, 0>(uh, a_wh, a_qh, gm, igm1, ro_lim, pr_lim, a_uh);
@@ -935,7 +913,7 @@ PIP_HD double collision_vjp(const double (&um)[8], const double (&uh)[5], const 
 // state of the cell (primitives by cq2pv).  Returns the candidate.
 PIP_HD double cfl_mhd_grad(const double (&u)[8], double gm, double ro_lim, double pr_lim, double sg,
                            double (&g)[8]) {
-  const double inv = rcp_(u[0]);
+  const double inv = 1.0 / u[0];
   const double v[3] = {u[1] * inv, u[2] * inv, u[3] * inv};
   const double kin = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const double bb = u[5] * u[5] + u[6] * u[6] + u[7] * u[7];
@@ -943,21 +921,21 @@ PIP_HD double cfl_mhd_grad(const double (&u)[8], double gm, double ro_lim, doubl
   const double pr = rmax(pr_raw, pr_lim);
   const double de = rmax(u[0], ro_lim);
   const double dm = rmax(de, kTiny);
-  const double cs2 = gm * pr * rcp_(dm), valf2 = bb * rcp_(dm);
-  const double vabs = root_(kin);
-  const double c = root_(cs2 + valf2);
+  const double cs2 = gm * pr / dm, valf2 = bb / dm;
+  const double vabs = rsqrt_(kin);
+  const double c = rsqrt_(cs2 + valf2);
   const double Dn = vabs + c;
-  const double cand = sg * rcp_(Dn);
+  const double cand = sg / Dn;
   for (int n = 0; n < 8; ++n) g[n] = 0.0;
-  const double a_Dn = -sg * rcp_(Dn * Dn);
-  const double a_w = c > 0.0 ? a_Dn * rcp_(2.0 * c) : 0.0;
-  double a_pr = gm * rcp_(dm) * a_w;
-  const double a_dm = -(cs2 + valf2) * rcp_(dm) * a_w;
-  double a_bb = a_w * rcp_(dm);
+  const double a_Dn = -sg / (Dn * Dn);
+  const double a_w = c > 0.0 ? a_Dn / (2.0 * c) : 0.0;
+  double a_pr = gm / dm * a_w;
+  const double a_dm = -(cs2 + valf2) / dm * a_w;
+  double a_bb = a_w / dm;
   double a_de = de >= kTiny ? a_dm : 0.0;
   double a_v[3] = {0, 0, 0};
   if (vabs > 0.0)
-    for (int k = 0; k < 3; ++k) a_v[k] = v[k] * rcp_(vabs) * a_Dn;
+    for (int k = 0; k < 3; ++k) a_v[k] = v[k] / vabs * a_Dn;
   const double a_prraw = pr_raw >= pr_lim ? a_pr : 0.0;
   double a_u0 = u[0] >= ro_lim ? a_de : 0.0;
   g[4] += (gm - 1.0) * a_prraw;
@@ -977,26 +955,26 @@ PIP_HD double cfl_mhd_grad(const double (&u)[8], double gm, double ro_lim, doubl
 // Gradient of cfl_hd_cell (Scheme_rot.f90:229-233).  Returns the candidate.
 PIP_HD double cfl_hd_grad(const double (&u)[5], double gm, double ro_lim, double pr_lim, double sg,
                           double (&g)[5]) {
-  const double inv = rcp_(u[0]);
+  const double inv = 1.0 / u[0];
   const double v[3] = {u[1] * inv, u[2] * inv, u[3] * inv};
   const double kin = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const double pr_raw = (gm - 1.0) * (u[4] - 0.5 * u[0] * kin);
   const double pr = rmax(pr_raw, pr_lim);
   const double de = rmax(u[0], ro_lim);
-  const double X = gm * pr * rcp_(de);
-  const double cs = root_(X);
+  const double X = gm * pr / de;
+  const double cs = rsqrt_(X);
   const double kc = rmax(kin, kTiny);
-  const double vabs = root_(kc);
+  const double vabs = rsqrt_(kc);
   const double Dn = vabs + cs;
-  const double cand = sg * rcp_(Dn);
+  const double cand = sg / Dn;
   for (int n = 0; n < 5; ++n) g[n] = 0.0;
-  const double a_Dn = -sg * rcp_(Dn * Dn);
-  const double a_X = cs > 0.0 ? a_Dn * rcp_(2.0 * cs) : 0.0;
-  const double a_pr = gm * rcp_(de) * a_X;
-  const double a_de = -X * rcp_(de) * a_X;
+  const double a_Dn = -sg / (Dn * Dn);
+  const double a_X = cs > 0.0 ? a_Dn / (2.0 * cs) : 0.0;
+  const double a_pr = gm / de * a_X;
+  const double a_de = -X / de * a_X;
   double a_v[3] = {0, 0, 0};
   if (kin >= kTiny)
-    for (int k = 0; k < 3; ++k) a_v[k] = v[k] * rcp_(vabs) * a_Dn;
+    for (int k = 0; k < 3; ++k) a_v[k] = v[k] / vabs * a_Dn;
   const double a_prraw = pr_raw >= pr_lim ? a_pr : 0.0;
   double a_u0 = u[0] >= ro_lim ? a_de : 0.0;
   g[4] += (gm - 1.0) * a_prraw;
