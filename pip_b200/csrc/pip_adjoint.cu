@@ -810,7 +810,7 @@ int pip_adj_create(const pip_params *p, int64_t max_steps, int checkpoint_every,
   a->p = *p;
   a->p.dx = a->p.dy = a->p.dz = nullptr;
   a->kp = k;
-  a->L = p->fp_exact ? &pip::launchers_exact() : &pip::launchers_fast();
+  a->L = &pip::launchers_of(*p);
   a->max_steps = max_steps;
   a->K = checkpoint_every > 0 ? checkpoint_every : 25;
   a->nseg_max = (int)((max_steps + a->K - 1) / a->K);

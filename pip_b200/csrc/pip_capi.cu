@@ -265,6 +265,7 @@ void build_kparams(pip_ctx *c) {
   k.ny = p.ndim == 2 ? p.jx - 2 * k.m1 : 1;
   k.nvm = p.nvar_m;
   k.imp = p.flag_pip_imp;
+  k.heat = p.flag_heat;
   k.ir = p.flag_ir != PIP_IR_NONE;
   k.ir_type = p.flag_ir_type;
   ir_law_constants(p, k);
@@ -335,6 +336,17 @@ void build_kparams(pip_ctx *c) {
 
 void pip::record_cuda_error(int code) { g_last_cuda_error = code; }
 
+// The reciprocal forms (pip_fp64_rcp.cu says why) for conduction and for the blocks that
+// pip_adj_create takes.
+static bool rcp_forms(const pip_params &p) {
+  if (p.flag_heat == 1) return true;
+  return p.precision == PIP_FP64 && p.flag_divb == 0 && p.flag_pip_imp == 0 &&
+         p.flag_ir == PIP_IR_NONE && p.flag_col == 1 && p.flag_resi == 0;
+}
+const pip::Launchers &pip::launchers_of(const pip_params &p) {
+  return p.fp_exact ? launchers_exact() : rcp_forms(p) ? launchers_rcp() : launchers_fast();
+}
+
 // Kernel parameters straight from a parameter block, for callers without a context: the
 // same validation and tables as pip_ctx_create, built on the stack (no allocation).  The
 // dx/dy pointers of the result are left null for the caller to point at device copies.
@@ -355,6 +367,7 @@ int pip::kparams_from_params(const pip_params *p, KParams *k) {
   k->ny = p->ndim == 2 ? p->jx - 2 * k->m1 : 1;
   k->nvm = p->nvar_m;
   k->imp = p->flag_pip_imp;
+  k->heat = p->flag_heat;
   k->ir = p->flag_ir != PIP_IR_NONE;
   k->ir_type = p->flag_ir_type;
   k->nc = (long long)p->ix * p->jx;
@@ -678,8 +691,7 @@ int pip_ctx_create(const pip_params *p, pip_ctx **out) {
   c->dz.assign(p->dz, p->dz + p->kx);
   c->p.dx = c->p.dy = c->p.dz = nullptr;
   build_kparams(c);
-  c->L = p->fp_exact ? &pip::launchers_exact()
-                     : p->flag_heat == 1 ? &pip::launchers_heat() : &pip::launchers_fast();
+  c->L = &pip::launchers_of(*p);
   c->mixed = p->precision == PIP_MIXED;
   auto fail = [&](cudaError_t e) {
     g_last_cuda_error = (int)e;

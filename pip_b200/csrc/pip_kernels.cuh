@@ -37,6 +37,7 @@ struct KParams {
   int irf;           // 1: set_IR type 1, rates frozen in irg between the time loop's set_IR calls
   int ir_type;       // IR energy form 0 (with the ionisation potential, set_IR type 4), 1 or 2
   int irn;           // set_IR type 4: the 6-level hydrogen model (FP64 form; irs = 4 as well)
+  int heat;          // implicit conduction follows the stages (flag_heat)
   long long nc;      // ix*jx
   double gm, ro_lim, pr_lim, ac, safety;
   double igm1;       // 1/(gm-1)
@@ -162,7 +163,7 @@ struct Launchers {
 };
 
 const Launchers &launchers_fast();
-const Launchers &launchers_heat();   // contexts with conduction: see pip_fp64_heat.cu
+const Launchers &launchers_rcp();    // see pip_fp64_rcp.cu
 const Launchers &launchers_exact();
 
 }  // namespace pip
@@ -215,6 +216,10 @@ void nlev_constants(NlevConst *k);
 // Validates a parameter block and fills the kernel parameters without allocating
 // (pip_capi.cu); dx and dy of the result are left null.
 int kparams_from_params(const pip_params *p, KParams *k);
+
+// The flavour of a parameter block's FP64 kernels (pip_capi.cu).  The context, the adjoint and
+// pip_step_noalloc all take it from here, so that their steps agree bit for bit.
+const Launchers &launchers_of(const pip_params &p);
 
 // FP32-mixed form (pip_mixed.cu): A = (hi, lo) FP32 pair, B = FP32 stage state.
 cudaError_t mixed_prepare();

@@ -58,7 +58,7 @@ extern "C" int pip_step_noalloc(const pip_params *p, double *U_dev, double dt, d
   if (k.nc > PIP_NOALLOC_MAX_CELLS || p->ix > PIP_NOALLOC_MAX_AXIS || p->jx > PIP_NOALLOC_MAX_AXIS)
     return PIP_ERR_PARAM;
   if (!(dt > 0.0) || !std::isfinite(dt) || !std::isfinite(cmax)) return PIP_ERR_PARAM;
-  const pip::Launchers &L = p->fp_exact ? pip::launchers_exact() : pip::launchers_fast();
+  const pip::Launchers &L = pip::launchers_of(*p);
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -71,8 +71,9 @@ extern "C" int pip_step_noalloc(const pip_params *p, double *U_dev, double dt, d
       void *ptr = nullptr;
       if ((e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch)) != cudaSuccess) return cuda_fail(e);
       if (!ptr) return PIP_ERR_CUDA;
-      // both FP64 flavours, so a later call with the other fp_exact also finds its limit set
+      // every FP64 flavour, so a later call with another block also finds its limit set
       if ((e = pip::launchers_fast().prepare(nullptr)) != cudaSuccess) return cuda_fail(e);
+      if ((e = pip::launchers_rcp().prepare(nullptr)) != cudaSuccess) return cuda_fail(e);
       if ((e = pip::launchers_exact().prepare(nullptr)) != cudaSuccess) return cuda_fail(e);
       g_scratch_addr[dev] = ptr;
     }

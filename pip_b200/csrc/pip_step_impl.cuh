@@ -1,8 +1,8 @@
 // pip_step_impl.cuh -- FP64 kernels of the two-fluid step, in three flavours:
 //   pip_fp64_fast.cu   FMA contraction, PIP_RCP and PIP_FAST: the forms of
 //                      pip_fp64_forms.cuh (the default build)
-//   pip_fp64_heat.cu   FMA contraction, PIP_RCP: the reciprocal forms of pip_physics.cuh, for
-//                      contexts with implicit conduction (see launch_stage)
+//   pip_fp64_rcp.cu    FMA contraction, PIP_RCP: the reciprocal forms of pip_physics.cuh, for
+//                      runs whose results hang on every rounding (see there)
 //   pip_fp64_exact.cu  -fmad=false: the literal forms, bitwise comparable with the CPU
 //                      restatement
 // PIP_FLAVOUR names the namespace and PIP_LAUNCHERS the table getter.
@@ -21,9 +21,10 @@
 #include "pip_physics.cuh"
 #include "pip_tma.cuh"
 
-// 1: the flavour of conduction contexts, 2D without resistivity
-#ifndef PIP_HEAT_ONLY
-#define PIP_HEAT_ONLY 0
+// 1: only the instances that rcp_forms (pip_capi.cu) leads to: no resistivity, and per-stage
+// coefficients in 2D only
+#ifndef PIP_RCP_ONLY
+#define PIP_RCP_ONLY 0
 #endif
 
 namespace pip {
@@ -1573,17 +1574,28 @@ constexpr size_t stage_smem_bytes() {
                            (S == 1 ? 2 * (NVM + 5) * 32 : 0));
 }
 
+// The instances of this flavour: of extra physics X, and of small tiles with it.
+template <int NDIM, int X>
+constexpr bool has_x() {
+  return !PIP_RCP_ONLY || X == 0 || (NDIM == 2 && X == 1);
+}
+template <int NVM, int X>
+constexpr bool has_small() {
+  return !PIP_RCP_ONLY || (X == 0 && NVM == 8);
+}
+
 template <int NDIM, int NVM, int STAGE, int X>
 static cudaError_t set_stage_attr_x() {
-  const cudaError_t e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 0>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)stage_smem_bytes<NDIM, NVM, X, 0>());
-#if !PIP_HEAT_ONLY
-  if (e == cudaSuccess)
-    return cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 1>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)stage_smem_bytes<NDIM, NVM, X, 1>());
-#endif
+  cudaError_t e = cudaSuccess;
+  if constexpr (has_x<NDIM, X>())
+    e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 0>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)stage_smem_bytes<NDIM, NVM, X, 0>());
+  if constexpr (has_small<NVM, X>())
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 1>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)stage_smem_bytes<NDIM, NVM, X, 1>());
   return e;
 }
 
@@ -1592,11 +1604,8 @@ static cudaError_t set_stage_attr() {
   cudaError_t e;
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 0>()) != cudaSuccess) return e;
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 1>()) != cudaSuccess) return e;
-#if !PIP_HEAT_ONLY
   if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 2>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 3>()) != cudaSuccess) return e;
-#endif
-  return cudaSuccess;
+  return set_stage_attr_x<NDIM, NVM, STAGE, 3>();
 }
 
 // Raises the dynamic shared-memory limit of the stage-kernel instances for p's dimension and
@@ -1604,12 +1613,10 @@ static cudaError_t set_stage_attr() {
 // that graph capture sees launches only.  Setting the limit loads the instance, about 1 ms.
 static cudaError_t prepare(const KParams *p) {
   cudaError_t e;
-#if !PIP_HEAT_ONLY
   if (!p || p->ndim == 1) {
     if ((e = set_stage_attr<1, 8, 1>()) != cudaSuccess) return e;
     if ((e = set_stage_attr<1, 8, 2>()) != cudaSuccess) return e;
   }
-#endif
   if (!p || (p->ndim == 2 && p->nvm == 8)) {
     if ((e = set_stage_attr<2, 8, 1>()) != cudaSuccess) return e;
     if ((e = set_stage_attr<2, 8, 2>()) != cudaSuccess) return e;
@@ -1630,19 +1637,19 @@ static cudaError_t prepare(const KParams *p) {
 #define PIP_SMALL_TILES 296
 #endif
 static bool small_tiles(const KParams &p) {
-#if PIP_HEAT_ONLY
-  return false;
-#else
+  // the flavour without every instance (has_small), whose conduction runs keep the large ones
+  if (PIP_RCP_ONLY && (p.heat || p.nvm != 8 || p.col_type || p.irl)) return false;
   if (p.ndim == 1) return (p.nx + Tile<1, 1>::TX - 1) / Tile<1, 1>::TX <= PIP_SMALL_TILES;
   return (long long)((p.nx + Tile<2, 1>::TX - 1) / Tile<2, 1>::TX) *
              ((p.ny + Tile<2, 1>::TY - 1) / Tile<2, 1>::TY) <= PIP_SMALL_TILES;
-#endif
 }
 
 template <int NDIM, int NVM, int STAGE, int X, int S>
 static cudaError_t launch_tiles(const KParams &p, const double *Us, const double *U0, double *Uo,
                                 DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                 const CUtensorMap *tm, int rows) {
+  if constexpr (!(S == 0 ? has_x<NDIM, X>() : has_small<NVM, X>())) return cudaErrorInvalidValue;
+  else {
   constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = tile_threads<NDIM, S>();
   const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
   if (NDIM == 1) rows = 0;
@@ -1664,6 +1671,7 @@ static cudaError_t launch_tiles(const KParams &p, const double *Us, const double
   cfg.numAttrs = rows == 0 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, stage_kernel<NDIM, NVM, STAGE, X, S>, p, Us, U0, Uo, ctrl, dt_mode,
                             epi, tm ? *tm : none, tm ? 1 : 0, rows);
+  }
 }
 
 template <int NDIM, int NVM, int STAGE, int S>
@@ -1675,15 +1683,10 @@ static cudaError_t launch_stage_t(const KParams &p, const double *Us, const doub
       return launch_tiles<NDIM, NVM, STAGE, 0, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
     case 1:
       return launch_tiles<NDIM, NVM, STAGE, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
-#if !PIP_HEAT_ONLY
     case 2:
       return launch_tiles<NDIM, NVM, STAGE, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
     default:
       return launch_tiles<NDIM, NVM, STAGE, 3, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
-#else
-    default:
-      return cudaErrorInvalidValue;
-#endif
   }
 }
 
@@ -1691,14 +1694,10 @@ template <int S>
 static cudaError_t launch_stage_s(const KParams &p, int stage, const double *Us, const double *U0,
                                   double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                   const CUtensorMap *tm, int rows) {
-#if PIP_HEAT_ONLY
-  if (p.ndim != 2) return cudaErrorInvalidValue;
-#else
   if (p.ndim == 1) {
     return stage == 1 ? launch_stage_t<1, 8, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0)
                       : launch_stage_t<1, 8, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, nullptr, 0);
   }
-#endif
   if (p.nvm == 9)
     return stage == 1 ? launch_stage_t<2, 9, 1, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
                       : launch_stage_t<2, 9, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
@@ -1711,13 +1710,11 @@ static cudaError_t launch_stage_s(const KParams &p, int stage, const double *Us,
 static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
                                 double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                 const CUtensorMap *tm, int rows) {
-#if !PIP_HEAT_ONLY
   if (small_tiles(p)) {
     if (rows == 0)
       return launch_stage_s<1>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, 0);
     tm = nullptr;
   }
-#endif
   return launch_stage_s<0>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 }
 
