@@ -1227,8 +1227,12 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   }
   if (STAGE == 2 && COL && p.col_type) exchanged_ghost_ac<NDIM, NVM, TX, TY, NTA>(p, Us, i0, j0, tid, by, nby);
   if (STAGE == 2 && s_epi == 2) {
-    if (RES && p.resi == 2) dtc = fmin(dtc, rb);  // the next step's cfl_resi
-    block_reduce_cfl<NTA, S == 1>(dtc, rhoc, grc, ctrl, s_slot);
+    if (RES && p.resi == 2) {
+      // the next step's cfl_resi: its bounds lie in every warp, not in those of the cells alone
+      block_reduce_cfl<NTA>(fmin(dtc, rb), rhoc, grc, ctrl, s_slot);
+    } else {
+      block_reduce_cfl<NTA, S == 1>(dtc, rhoc, grc, ctrl, s_slot);
+    }
   }
   if (S == 1 && edge) {
     __syncthreads();
