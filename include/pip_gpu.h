@@ -468,8 +468,8 @@ int pip_dev_stage(pip_ctx *ctx, int stage);
 
 /* The y exchange overlapped with the stage (2D; no counterpart in the reference, whose
  * mpi_bnd runs after the whole stage).  pip_dev_stage_split(ctx, k, &bs) queues stage k
- * as two launches: the first and the last row of tiles -- every cell the exchange sends --
- * on a high-priority stream of the context, returned in bs, and the rows between them on
+ * as two launches: the rows of tiles at both ends that hold the cells the exchange sends on a
+ * high-priority stream of the context, returned in bs, and the rows between them on
  * the context stream, concurrently; the context stream then waits for the boundary rows.
  * Together they equal pip_dev_stage(ctx, k) bit for bit.  The caller records an event on
  * bs right after the call and runs the exchange (pack, transfer, unpack) on a stream of its

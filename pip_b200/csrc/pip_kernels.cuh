@@ -126,8 +126,8 @@ struct DevCtrl {
 struct Launchers {
   cudaError_t (*prepare)(const KParams *p);   // null: every grid's instances
   // tm: the TMA map of Us for the 2D tiles (tile_map), or null for per-thread loads.  rows
-  // (2D): 0 every tile row; 1 the first and the last tile row (those a y-halo exchange
-  // sends); 2 the rows between them.  A stage launched as 1 then 2 equals one launch of 0.
+  // (2D): 0 every tile row; 1 the tile rows that a y-halo exchange sends from; 2 the rows
+  // between them (pip_rows.cuh).  A stage launched as 1 then 2 equals one launch of 0.
   cudaError_t (*stage)(const KParams &p, int stage, const double *Us, const double *U0, double *Uo,
                        DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s, const CUtensorMap *tm,
                        int rows);

@@ -20,6 +20,7 @@
 #include "pip_mixed_cell.cuh"
 #include "pip_physics.cuh"
 #include "pip_mixed_tile.cuh"
+#include "pip_rows.cuh"
 #include "pip_tma.cuh"
 
 namespace pip {
@@ -122,10 +123,9 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
   __shared__ int s_exit, s_epi, s_slot;
 
   const int tid = threadIdx.x;
-  // tile row: every row (rows 0), the first and the last (1), the rows between them (2)
+  // tile row: every row (rows 0), those a halo exchange sends (1), the rows between them (2)
   const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
-  const int by = NDIM == 1 || rows == 0 ? (int)blockIdx.y
-                 : rows == 1 ? (blockIdx.y == 0 ? 0 : nby - 1) : (int)blockIdx.y + 1;
+  const int by = NDIM == 1 ? 0 : tile_row(rows, (int)blockIdx.y, (int)gridDim.y, nby);
   const bool block0 = blockIdx.x == 0 && by == 0;
   const int i0 = p.m0 + blockIdx.x * TX;
   const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
@@ -310,10 +310,9 @@ static cudaError_t launch_t(const KParams &p, const float *Us, const float *U0hi
                             float *Ohi, float *Olo, DevCtrl *ctrl, int dt_mode, int epi,
                             cudaStream_t s, const CUtensorMap *tm, int rows) {
   constexpr int TX = Tile<NDIM>::TX, TY = Tile<NDIM>::TY, NT = Tile<NDIM>::NT;
-  const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
   if (NDIM == 1) rows = 0;
-  const int gy = rows == 0 ? nby : rows == 1 ? (nby < 2 ? nby : 2) : nby - 2;
-  if (gy <= 0) return cudaSuccess;   // no rows between the first and the last
+  const int gy = NDIM == 2 ? tile_rows(rows, p.ny, TY, p.m1) : 1;
+  if (gy <= 0) return cudaSuccess;   // no rows between those that are sent
   CUtensorMap none;
   std::memset(&none, 0, sizeof none);
   cudaLaunchConfig_t cfg = {};

@@ -19,6 +19,7 @@
 #include "pip_ghosts.cuh"
 #include "pip_kernels.cuh"
 #include "pip_physics.cuh"
+#include "pip_rows.cuh"
 #include "pip_tma.cuh"
 
 // 1: only the instances that rcp_forms (pip_capi.cu) leads to: no resistivity, and per-stage
@@ -633,11 +634,10 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   __shared__ __align__(8) unsigned long long s_bar;
 
   const int tid = threadIdx.x;
-  // tile row of this CTA: every row (rows 0), the first and the last (1: the rows a halo
-  // exchange sends, launched first), or the rows between them (2)
+  // tile row of this CTA: every row (rows 0), those with the rows a halo exchange sends (1,
+  // launched first), or the rows between them (2)
   const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
-  const int by = NDIM == 1 || rows == 0 ? (int)blockIdx.y
-                 : rows == 1 ? (blockIdx.y == 0 ? 0 : nby - 1) : (int)blockIdx.y + 1;
+  const int by = NDIM == 1 ? 0 : tile_row(rows, (int)blockIdx.y, (int)gridDim.y, nby);
   const bool block0 = blockIdx.x == 0 && by == 0;
   const int i0 = p.m0 + blockIdx.x * TX;
   const int j0 = NDIM == 2 ? p.m1 + by * TY : 0;
@@ -1655,10 +1655,9 @@ static cudaError_t launch_tiles(const KParams &p, const double *Us, const double
   if constexpr (!(S == 0 ? has_x<NDIM, X>() : has_small<NVM, X>())) return cudaErrorInvalidValue;
   else {
   constexpr int TX = Tile<NDIM, S>::TX, TY = Tile<NDIM, S>::TY, NT = tile_threads<NDIM, S>();
-  const int nby = NDIM == 2 ? (p.ny + TY - 1) / TY : 1;
   if (NDIM == 1) rows = 0;
-  const int gy = rows == 0 ? nby : rows == 1 ? (nby < 2 ? nby : 2) : nby - 2;
-  if (gy <= 0) return cudaSuccess;   // no rows between the first and the last
+  const int gy = NDIM == 2 ? tile_rows(rows, p.ny, TY, p.m1) : 1;
+  if (gy <= 0) return cudaSuccess;   // no rows between those that are sent
   CUtensorMap none;
   std::memset(&none, 0, sizeof none);
   cudaLaunchConfig_t cfg = {};
