@@ -1708,17 +1708,13 @@ static cudaError_t launch_stage_s(const KParams &p, int stage, const double *Us,
                     : launch_stage_t<2, 8, 2, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 }
 
-// The small tiles take whole stages only: the rows of a split stage are rows of the large
-// ones, whose map (tile_map makes one for the tiles of whole stages) such a context lacks.
+// (A split stage's rows are rows of the same tiles: tile_map makes one map a grid, and the two
+// launches agree with a whole stage because they are the same instance.)
 static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
                                 double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                 const CUtensorMap *tm, int rows) {
-  if (small_tiles(p)) {
-    if (rows == 0)
-      return launch_stage_s<1>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, 0);
-    tm = nullptr;
-  }
-  return launch_stage_s<0>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
+  return small_tiles(p) ? launch_stage_s<1>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
+                        : launch_stage_s<0>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 }
 
 template <int S>
