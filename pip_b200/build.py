@@ -21,7 +21,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           "-Xcompiler", "-Wno-unknown-pragmas", "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]
 EXTRA_FLAGS = {
-    "pip_fp64_exact.cu": ["-fmad=false"],
+    **{"pip_fp64_exact%s.cu" % x: ["-fmad=false"] for x in ("", "_x0", "_x1", "_x2", "_x3")},
     "pip_mixed.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "pip_ensemble.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
 }

@@ -124,7 +124,8 @@ struct DevCtrl {
 
 // Host launchers (one set per arithmetic flavour).
 struct Launchers {
-  cudaError_t (*prepare)(const KParams *p);   // null: every grid's instances
+  // limits of the instances that p launches (null: every grid's without extra physics)
+  cudaError_t (*prepare)(const KParams *p);
   // tm: the TMA map of Us for the 2D tiles (tile_map), or null for per-thread loads.  rows
   // (2D): 0 every tile row; 1 the tile rows that a y-halo exchange sends from; 2 the rows
   // between them (pip_rows.cuh).  A stage launched as 1 then 2 equals one launch of 0.
@@ -161,6 +162,23 @@ struct Launchers {
   cudaError_t (*nlev_rates_cfl)(const KParams &p, const double *U, DevCtrl *ctrl, int slot,
                                 cudaStream_t s);
 };
+
+// The stage kernels of one extra physics X of a flavour (Launchers' prepare and stage), each X in
+// a file of its own.
+struct StageSet {
+  cudaError_t (*prepare)(const KParams *p);
+  cudaError_t (*stage)(const KParams &p, int stage, const double *Us, const double *U0, double *Uo,
+                       DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s, const CUtensorMap *tm,
+                       int rows);
+};
+const StageSet &stages_fast_x0();
+const StageSet &stages_fast_x1();
+const StageSet &stages_fast_x2();
+const StageSet &stages_fast_x3();
+const StageSet &stages_exact_x0();
+const StageSet &stages_exact_x1();
+const StageSet &stages_exact_x2();
+const StageSet &stages_exact_x3();
 
 const Launchers &launchers_fast();
 const Launchers &launchers_rcp();    // see pip_fp64_rcp.cu

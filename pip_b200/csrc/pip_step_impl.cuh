@@ -7,6 +7,12 @@
 //                      restatement
 // PIP_FLAVOUR names the namespace and PIP_LAUNCHERS the table getter.
 //
+// The first launch of a kernel loads the module of its file, about 0.5 ms for each stage-kernel
+// instance in it.  So the instances of the fast and the exact flavour lie in a file for each extra
+// physics X (PIP_STAGE_X; pip_fp64_fast_x0.cu and so on), and a context loads the X it
+// launches: with all of them in one file the first context of a process took 28 ms (256x256,
+// alpha_c per cell), so 8, and its first cfl 2 more.
+//
 // Layout in HBM: one array of NV = nvm + 5 planes, each plane the Fortran
 // (ix,jx) slab with ghosts (x fastest): ion planes 0..nvm-1 (ro, mx, my, mz, en, bx, by,
 // bz[, psi]) then neutral planes nvm..nvm+4 (ro, mx, my, mz, en).  A step uses two such
@@ -27,6 +33,17 @@
 #ifndef PIP_RCP_ONLY
 #define PIP_RCP_ONLY 0
 #endif
+// Whether this file holds stage-kernel instances, and everything else
+#if defined(PIP_STAGE_X)
+#define PIP_HAS_STAGES 1
+#define PIP_HAS_REST 0
+#else
+#define PIP_HAS_STAGES PIP_RCP_ONLY
+#define PIP_HAS_REST 1
+#define PIP_STAGE_X 0
+#endif
+#define PIP_CAT2(a, b) a##b
+#define PIP_CAT(a, b) PIP_CAT2(a, b)
 
 namespace pip {
 namespace PIP_FLAVOUR {
@@ -1273,6 +1290,7 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
   }
 }
 
+#if PIP_HAS_REST
 // cfl (Scheme_rot.f90:183-213) as a standalone pass over every cell: cq2pv rewrite of
 // both species in place, CFL candidates of interior cells, rho*alpha_c and IR maxima of all
 // cells into reduction slot `slot`.  The default build notes in ctrl->floored that a floor acted.
@@ -1565,6 +1583,7 @@ __global__ void nan_kernel(const double *__restrict__ U, long long n, int *flag)
 }
 
 #include "pip_nlevel_impl.cuh"
+#endif  // PIP_HAS_REST
 
 // ---------------------------------------------------------------- host launchers
 
@@ -1578,58 +1597,14 @@ constexpr size_t stage_smem_bytes() {
                            (S == 1 ? 2 * (NVM + 5) * 32 : 0));
 }
 
-// The instances of this flavour: of extra physics X, and of small tiles with it.
+// The instances of this file: of extra physics X, and of small tiles with it.
 template <int NDIM, int X>
-constexpr bool has_x() {
-  return !PIP_RCP_ONLY || X == 0 || (NDIM == 2 && X == 1);
+static constexpr bool has_x() {
+  return PIP_RCP_ONLY ? X == 0 || (NDIM == 2 && X == 1) : X == PIP_STAGE_X;
 }
 template <int NVM, int X>
-constexpr bool has_small() {
-  return !PIP_RCP_ONLY || (X == 0 && NVM == 8);
-}
-
-template <int NDIM, int NVM, int STAGE, int X>
-static cudaError_t set_stage_attr_x() {
-  cudaError_t e = cudaSuccess;
-  if constexpr (has_x<NDIM, X>())
-    e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stage_smem_bytes<NDIM, NVM, X, 0>());
-  if constexpr (has_small<NVM, X>())
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(stage_kernel<NDIM, NVM, STAGE, X, 1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)stage_smem_bytes<NDIM, NVM, X, 1>());
-  return e;
-}
-
-template <int NDIM, int NVM, int STAGE>
-static cudaError_t set_stage_attr() {
-  cudaError_t e;
-  if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 0>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 1>()) != cudaSuccess) return e;
-  if ((e = set_stage_attr_x<NDIM, NVM, STAGE, 2>()) != cudaSuccess) return e;
-  return set_stage_attr_x<NDIM, NVM, STAGE, 3>();
-}
-
-// Raises the dynamic shared-memory limit of the stage-kernel instances for p's dimension and
-// ion planes (p null: of every instance) on the current device; called once per context so
-// that graph capture sees launches only.  Setting the limit loads the instance, about 1 ms.
-static cudaError_t prepare(const KParams *p) {
-  cudaError_t e;
-  if (!p || p->ndim == 1) {
-    if ((e = set_stage_attr<1, 8, 1>()) != cudaSuccess) return e;
-    if ((e = set_stage_attr<1, 8, 2>()) != cudaSuccess) return e;
-  }
-  if (!p || (p->ndim == 2 && p->nvm == 8)) {
-    if ((e = set_stage_attr<2, 8, 1>()) != cudaSuccess) return e;
-    if ((e = set_stage_attr<2, 8, 2>()) != cudaSuccess) return e;
-  }
-  if (!p || (p->ndim == 2 && p->nvm == 9)) {
-    if ((e = set_stage_attr<2, 9, 1>()) != cudaSuccess) return e;
-    if ((e = set_stage_attr<2, 9, 2>()) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+static constexpr bool has_small() {
+  return PIP_RCP_ONLY ? X == 0 && NVM == 8 : X == PIP_STAGE_X;
 }
 
 // Whether a grid takes the small tiles (Tile<., 1>): while they all run at once, two a SM.
@@ -1646,6 +1621,55 @@ static bool small_tiles(const KParams &p) {
   if (p.ndim == 1) return (p.nx + Tile<1, 1>::TX - 1) / Tile<1, 1>::TX <= PIP_SMALL_TILES;
   return (long long)((p.nx + Tile<2, 1>::TX - 1) / Tile<2, 1>::TX) *
              ((p.ny + Tile<2, 1>::TY - 1) / Tile<2, 1>::TY) <= PIP_SMALL_TILES;
+}
+
+// The extra physics of a parameter block (the X of its instances).
+static int extra_physics(const KParams &p) {
+  return (p.col_type || p.irl ? 1 : 0) | (p.resi ? 2 : 0);
+}
+
+#if PIP_HAS_STAGES
+template <int NDIM, int NVM, int X, int S>
+static cudaError_t set_limits_s() {
+  if constexpr (S == 0 ? has_x<NDIM, X>() : has_small<NVM, X>()) {
+    const int bytes = (int)stage_smem_bytes<NDIM, NVM, X, S>();
+    const cudaError_t e = cudaFuncSetAttribute(
+        stage_kernel<NDIM, NVM, 1, X, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(stage_kernel<NDIM, NVM, 2, X, S>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  }
+  return cudaSuccess;
+}
+template <int NDIM, int NVM, int X>
+static cudaError_t set_limits_x(const KParams *p) {
+  cudaError_t e = cudaSuccess;
+  if (!p || !small_tiles(*p)) e = set_limits_s<NDIM, NVM, X, 0>();
+  if (e == cudaSuccess && (!p || small_tiles(*p))) e = set_limits_s<NDIM, NVM, X, 1>();
+  return e;
+}
+template <int NDIM, int NVM>
+static cudaError_t set_limits(const KParams *p) {
+  switch (p ? extra_physics(*p) : 0) {
+    case 0: return set_limits_x<NDIM, NVM, 0>(p);
+    case 1: return set_limits_x<NDIM, NVM, 1>(p);
+    case 2: return set_limits_x<NDIM, NVM, 2>(p);
+    default: return set_limits_x<NDIM, NVM, 3>(p);
+  }
+}
+
+// Raises the dynamic shared-memory limit of the two stage-kernel instances that p's grid and
+// physics launch (p null: of every grid's without extra physics) on the current device; called
+// once per context so that graph capture sees launches only.
+static cudaError_t prepare(const KParams *p) {
+  cudaError_t e;
+  if (!p || p->ndim == 1)
+    if ((e = set_limits<1, 8>(p)) != cudaSuccess) return e;
+  if (!p || (p->ndim == 2 && p->nvm == 8))
+    if ((e = set_limits<2, 8>(p)) != cudaSuccess) return e;
+  if (!p || (p->ndim == 2 && p->nvm == 9))
+    if ((e = set_limits<2, 9>(p)) != cudaSuccess) return e;
+  return cudaSuccess;
 }
 
 template <int NDIM, int NVM, int STAGE, int X, int S>
@@ -1681,7 +1705,7 @@ template <int NDIM, int NVM, int STAGE, int S>
 static cudaError_t launch_stage_t(const KParams &p, const double *Us, const double *U0, double *Uo,
                                   DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
                                   const CUtensorMap *tm, int rows) {
-  switch ((p.col_type || p.irl ? 1 : 0) | (p.resi ? 2 : 0)) {
+  switch (extra_physics(p)) {
     case 0:
       return launch_tiles<NDIM, NVM, STAGE, 0, S>(p, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
     case 1:
@@ -1716,7 +1740,24 @@ static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, c
   return small_tiles(p) ? launch_stage_s<1>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows)
                         : launch_stage_s<0>(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
 }
+#else
+static const StageSet &stages(const KParams *p) {
+  switch (p ? extra_physics(*p) : 0) {
+    case 0: return PIP_CAT(PIP_CAT(stages_, PIP_FLAVOUR), _x0)();
+    case 1: return PIP_CAT(PIP_CAT(stages_, PIP_FLAVOUR), _x1)();
+    case 2: return PIP_CAT(PIP_CAT(stages_, PIP_FLAVOUR), _x2)();
+    default: return PIP_CAT(PIP_CAT(stages_, PIP_FLAVOUR), _x3)();
+  }
+}
+static cudaError_t prepare(const KParams *p) { return stages(p).prepare(p); }
+static cudaError_t launch_stage(const KParams &p, int stage, const double *Us, const double *U0,
+                                double *Uo, DevCtrl *ctrl, int dt_mode, int epi, cudaStream_t s,
+                                const CUtensorMap *tm, int rows) {
+  return stages(&p).stage(p, stage, Us, U0, Uo, ctrl, dt_mode, epi, s, tm, rows);
+}
+#endif  // PIP_HAS_STAGES
 
+#if PIP_HAS_REST
 template <int S>
 static bool tile_map_s(const KParams &p, const double *U, CUtensorMap *map) {
   constexpr int TX = Tile<2, S>::TX, RY = Tile<2, S>::TY + 2 * kH;
@@ -1843,8 +1884,16 @@ static cudaError_t launch_nan(const KParams &p, const double *U, int *flag, cuda
   return cudaGetLastError();
 }
 
+#endif  // PIP_HAS_REST
+
 }  // namespace PIP_FLAVOUR
 
+#if !PIP_HAS_REST
+const StageSet &PIP_CAT(PIP_CAT(stages_, PIP_FLAVOUR), PIP_CAT(_x, PIP_STAGE_X))() {
+  static const StageSet S = {PIP_FLAVOUR::prepare, PIP_FLAVOUR::launch_stage};
+  return S;
+}
+#else
 const Launchers &PIP_LAUNCHERS() {
   static const Launchers L = {PIP_FLAVOUR::prepare,       PIP_FLAVOUR::launch_stage,
                               PIP_FLAVOUR::launch_cfl,    PIP_FLAVOUR::launch_ghosts,
@@ -1856,5 +1905,6 @@ const Launchers &PIP_LAUNCHERS() {
                               PIP_FLAVOUR::launch_nlev_rates_cfl};
   return L;
 }
+#endif
 
 }  // namespace pip
