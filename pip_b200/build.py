@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from typing import List
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -51,8 +52,8 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= newest:
         return LIB
     os.makedirs(BUILD, exist_ok=True)
-    objs = []
-    for src in sources():
+
+    def compile_one(src: str) -> str:
         obj = os.path.join(BUILD, src[:-3] + ".o")
         cmd = [nvcc()] + ARCH + COMMON + EXTRA_FLAGS.get(src, [])
         if ptxas_info:
@@ -61,7 +62,10 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(obj)
+        return obj
+
+    with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(compile_one, sources()))
     tmp = LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-shared", "-o", tmp] + objs
     subprocess.run(cmd, check=True)
