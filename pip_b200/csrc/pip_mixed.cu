@@ -195,7 +195,7 @@ stage_kernel(const __grid_constant__ KParams p, const float *__restrict__ Us, co
     }
   }
   if (STAGE == 2 && dt_mode == 1 && block0 && tid == 0) {
-    // end of step; no block of stage 2 reads what changes here
+    // end of step; the other blocks load only status of this, and ask whether it is 5
     ctrl->time = ctrl->time_next;
     ctrl->step = ctrl->step + 1;
     if (ctrl->last) ctrl->done = 1;

@@ -13,11 +13,13 @@ namespace mixed {
 
 // The source's results round to the FP32 stage state, and where one lands next to a rounding
 // boundary a last bit moves the state by 1e-7 and the fluxes with it (in one of about fifteen
-// 1024x1024 runs of 100 steps an exchange that differed by rounding did).  So its quotients are the
-// correctly rounded ones, from one reciprocal a denominator: q = a y, corrected by its
-// residual, q + (a - x q) y, rounds as a / x does (Markstein, IBM J. Res. Dev. 34, 1990, with y
-// = 1/x to within an ulp), in three operations and without the division's scaling and branches.
-// For normal operands and quotients; y = rcp_(x) or 1/x.
+// 1024x1024 runs of 100 steps an exchange that differed by rounding did).  So its quotients are
+// corrected ones, from one reciprocal a denominator: q = a y, then q + (a - x q) y (the last
+// step of Markstein's division, IBM J. Res. Dev. 34, 1990), in three operations and without the
+// division's scaling and branches.  His theorem asks for the correctly rounded reciprocal; with
+// y = rcp_(x), right to an ulp, quotients very close to a rounding boundary are not covered.
+// None of 2^30 sampled operand pairs differs from a / x (tests/div_check.cu).  For normal
+// operands and quotients; y = rcp_(x) or 1/x.
 __device__ __forceinline__ double div_rn(double a, double x, double y) {
   const double q = __dmul_rn(a, y);
   return fma(fma(-x, q, a), y, q);

@@ -818,7 +818,10 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     ctrl->skip = 0;
     ctrl->floored = 0;
     if (dt_mode == 1) {
-      // loop bookkeeping of main.f90:31,58 for this step (no block of stage 1 reads these)
+      // loop bookkeeping of main.f90:31,58 for this step.  Other blocks of this stage may load
+      // some of these words while they change, and drop what they loaded: dt and cmax, which
+      // dt_mode 1 forms anew, and the slot that is reset, which is not the step's (finalize_dt
+      // loads both).  No block of this stage loads the others.
       const long long st = ctrl->step;
       ctrl->dt = dt;
       ctrl->cmax = cmax;
@@ -836,8 +839,9 @@ stage_kernel(const __grid_constant__ KParams p, const double *__restrict__ Us, c
     }
   }
   if (STAGE == 2 && dt_mode == 1 && !(RES && p.resi == 2) && block0 && control) {
-    // end of step: time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636); no
-    // block of stage 2 reads what changes here
+    // end of step: time += dt and stop_sim's dt check (main.f90:58-66, IO_rot.f90:636).  Of the
+    // words that change here the other blocks of stage 2 load status alone, and ask only
+    // whether it is 5, which it does not become here.
     ctrl->time = ctrl->time_next;
     ctrl->step = ctrl->step + 1;
     if (ctrl->last) ctrl->done = 1;
