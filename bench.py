@@ -36,7 +36,8 @@ alpha_c = 1e3, Dedner cleaning, CFL 0.3) with synthetic initial data.
 * conduction: the 2048x1024 partially ionised Kelvin-Helmholtz run with ionisation/
   recombination and implicit anisotropic conduction (BiCGstab to 1e-10), 1000 steps, plain
   FP64 and FP32-mixed (FP32 inner solve with FP64 iterative refinement): ms per step,
-  iterations per step, solver time and GB/s per iteration, mixed-vs-FP64 L1.
+  iterations per step, time and GB/s of an iteration (against the same run with kapper = 0),
+  mixed-vs-FP64 L1.
 * alpha_c_per_cell, resistivity, ionisation_recombination: the FP64 OT step with
   flag_col=5 (set_collisional col_type 4: alpha_c from both temperatures and the drift,
   recomputed at every RK stage), with flag_resi=1, eta_0=1e-4 (resistive_flux on every

@@ -11,7 +11,7 @@
 //   moved in every shock tube (1 % of its norm, in the feet of the waves), beside open ends and
 //   walls (1e-4), and in 18 of 120 runs from a uniform start (single entries by 8e-3).  The
 //   adjoint's forward is pip_run bit for bit, so pip_run takes these forms for such blocks too:
-//   1D 1024 cells 11.7 us a step (8.2 with the other forms, 27.3 before the small tiles).
+//   1D 1024 cells 11.2 us a step (8.0 with the other forms, 26.1 before the small tiles).
 #define PIP_FLAVOUR rcp
 #define PIP_RCP 1
 #define PIP_FAST 0

@@ -1615,7 +1615,9 @@ static constexpr bool has_small() {
 // us a step, small | large tiles: 2D 64x64 10.8 | 17.1, 96x96 (288 small tiles) 12.0 | 17.0,
 // 112x96 (336) 18.6 | 17.0, 128x128 19.6 | 17.1, 256x256 59.8 | 25.6; 1D 1024 cells 9.0 | 12.1,
 // 8192 (265) 10.4 | 12.1, 65536 26.2 | 18.1 (without the control warp, which took 64x64 to 10.0 and
-// 1024 cells to 8.2).
+// 1024 cells to 8.2).  In the reciprocal forms (pip_fp64_rcp.cu): 64x64 15.6 | 23.2, 96x96 16.3 | 23.1,
+// 112x96 25.2 | 22.8, 256x256 81.3 | 31.8; 1D 1024 cells 11.2 | 18.4, 8192 12.6 | 19.1, 65536
+// 39.2 | 24.5.
 #ifndef PIP_SMALL_TILES
 #define PIP_SMALL_TILES 296
 #endif
