@@ -17,8 +17,8 @@
 // Measured on a B200, per step of two stage launches, the literal forms -> these, nothing else
 // changed: Orszag-Tang 1024^2 0.551 -> 0.370 ms; 517x333 with walls and the exponential
 // collisions 124 -> 85 us; 1024 cells in 1D 27.3 -> 20.5 us (a chain of dependent operations
-// there).  With the other changes of the stage kernels 0.310 ms, 67 us and 8.2 us (a tube with the
-// exponential exchange; the plain one runs the forms of pip_fp64_rcp.cu).  Error of the
+// there).  With the other changes of the stage kernels 0.310 ms, 67 us and 8.2 us (that tube now runs
+// the forms of pip_fp64_rcp.cu, 11.2 us).  Error of the
 // state against 64-bit torch after 100 steps: 3.8e-15 -> 3.2e-15.
 #pragma once
 
